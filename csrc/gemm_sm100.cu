@@ -84,10 +84,13 @@ struct GemmParams {
   // (consecutive CTAs share the WEIGHT tile: for a vocabulary matrix larger than L2 and many row tiles, each
   // weight tile then comes from HBM once instead of once per row tile)
   int m_fast;
-  // Grouped mode: a row tile with at most this many rows left loads its activations through the second tensor map,
-  // whose box holds only that many rows (0 = always the 128-row box).  With ~8 rows per expert (MoE decode) a
-  // 128-row box would make the activations half of every stage's bytes although almost none of its rows are used;
-  // the accumulator rows beyond the box read stale shared memory and are never stored.
+  // A row tile with at most this many rows left loads its activations through the second tensor map, whose box holds
+  // only that many rows (0 = always the 128-row box); the accumulator rows beyond the box read stale shared memory
+  // and are never stored.  Grouped mode: with ~8 rows per expert (MoE decode) a 128-row box would make the
+  // activations half of every stage's bytes although almost none of its rows are used.  Otherwise it is M % 128, so
+  // that the last row tile's box ends with the matrix: a box that lies mostly past the end is slow, because every CTA
+  // waits for its zero fill (4096 x 24576 weights at 1 row, 128-row box against 1-row box: 69.1 against 40.2 us per
+  // launch, 4096 x 6144 at 8 rows 24.2 against 15.5, 4096 x 151936 at 1 row 276 against 203; equal from 16 rows on).
   int a_small_rows;
   // EPI_INPROJ (fused input projections of a parallel block): columns below n_raw (a multiple of 128) are stored as
   // fp32 to C; the rest pass through `act` and go to C2 as bf16.  ACT_GELU_GLU: every 128 weight rows hold 64 gate rows
@@ -271,31 +274,38 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                        p.sfa + static_cast<size_t>(m0 / 128) * sf_row + static_cast<size_t>(kb) * 2048, 2048, &full_bar[s]);
       };
       // bytes a stage receives: the activation box shrinks for a row tile with few rows left (grouped mode)
-      auto small_tile = [&](int m_tile) { return p.a_small_rows > 0 && m_end - m_tile <= p.a_small_rows; };
-      auto stage_bytes = [&](bool small) {
-        return static_cast<uint32_t>(small ? S::kStage - S::kStageA + p.a_small_rows * BK * 2 : S::kStage);
+      auto box_rows = [&](int m) {       // rows of the activation box of the row tile at m (0: no rows left, MT == 2 only)
+        if (MT == 2 && m >= m_end) return 0;
+        return p.a_small_rows > 0 && m_end - m <= p.a_small_rows ? p.a_small_rows : BM;
       };
-      const bool small0 = small_tile(m0);
+      auto stage_bytes = [&](int m_tile) {
+        int rows = box_rows(m_tile);
+        if constexpr (MT == 2) rows += box_rows(m_tile + BM);
+        return static_cast<uint32_t>(S::kStage - S::kStageA + rows * BK * 2);
+      };
+      auto load_a = [&](int s, int x, int m_tile) {
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          const int rows = box_rows(m_tile + mt * BM);
+          if (rows > 0)
+            tma_load_2d(smem + s * S::kStage + mt * (BM * BK * 2), rows == BM ? &tmA : &tmA2, &full_bar[s], x, m_tile + mt * BM);
+        }
+      };
+      const uint32_t bytes0 = stage_bytes(m0);
       for (int i = 0; i < pre; ++i) {
-        mbar_expect_tx(&full_bar[i], stage_bytes(small0));
+        mbar_expect_tx(&full_bar[i], bytes0);
         tma_load_2d(smem + i * S::kStage + S::kStageA, &tmW, &full_bar[i], (kb_begin + i) * kXStep, wn0);
         load_sfw(i, kb_begin + i);
       }
       pdl_wait();
       for (int i = 0; i < pre; ++i) {
-        if (small0) {
-          tma_load_2d(smem + i * S::kStage, &tmA2, &full_bar[i], ax0 + (kb_begin + i) * kXStep, m0);
-        } else {
-#pragma unroll
-          for (int mt = 0; mt < MT; ++mt)
-            tma_load_2d(smem + i * S::kStage + mt * (BM * BK * 2), &tmA, &full_bar[i], ax0 + (kb_begin + i) * kXStep, m0 + mt * BM);
-        }
+        load_a(i, ax0 + (kb_begin + i) * kXStep, m0);
         load_sfa(i, kb_begin + i);
       }
       bool p_ok = true;
       for (int tj = 0; tj < n_tiles_cta && p_ok; ++tj) {
         const int m_tile = m_first + tj * tile_step;
-        const bool small = small_tile(m_tile);
+        const uint32_t bytes = stage_bytes(m_tile);
         for (int i = (tj == 0 ? pre : 0); i < nkb; ++i) {
           const int g = tj * nkb + i;              // running k-block count of this CTA
           const int s = g % kStages;
@@ -303,15 +313,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             const uint32_t ph = (g / kStages) & 1;
             if (!mbar_wait(&empty_bar[s], ph ^ 1, p.status, kTimeoutEmpty)) { p_ok = false; break; }
           }
-          mbar_expect_tx(&full_bar[s], stage_bytes(small));
+          mbar_expect_tx(&full_bar[s], bytes);
           tma_load_2d(smem + s * S::kStage + S::kStageA, &tmW, &full_bar[s], (kb_begin + i) * kXStep, wn0);
-          if (small) {
-            tma_load_2d(smem + s * S::kStage, &tmA2, &full_bar[s], ax0 + (kb_begin + i) * kXStep, m_tile);
-          } else {
-#pragma unroll
-            for (int mt = 0; mt < MT; ++mt)
-              tma_load_2d(smem + s * S::kStage + mt * (BM * BK * 2), &tmA, &full_bar[s], ax0 + (kb_begin + i) * kXStep, m_tile + mt * BM);
-          }
+          load_a(s, ax0 + (kb_begin + i) * kXStep, m_tile);
           load_sfw(s, kb_begin + i);
           load_sfa(s, kb_begin + i);
         }
@@ -1076,6 +1080,15 @@ static int make_map_u8(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t 
   return r == CUDA_SUCCESS ? 0 : -2;
 }
 
+// Activation maps of a launch over M rows: full 128-row boxes, and the box of the last row tile (GemmParams::a_small_rows)
+struct ActMaps { CUtensorMap full, last; };
+static int make_act_maps(ActMaps* m, GemmParams* p, const void* A, uint64_t cols, uint64_t ld, bool u8) {
+  auto make = u8 ? make_map_u8 : make_map;
+  p->a_small_rows = p->M % BM;
+  if (make(&m->full, A, p->M, cols, ld, BM)) return -1;
+  return p->a_small_rows > 0 ? make(&m->last, A, p->M, cols, ld, p->a_small_rows) : 0;
+}
+
 template <int BN, int EPI, int BUDGET_KB, bool FP4 = false, int MT = 1>
 static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tw, const GemmParams& p, int split, bool pdl,
                        cudaStream_t stream, int groups = 0, int group_m_tiles = 0, const CUtensorMap* ta_small = nullptr) {
@@ -1109,8 +1122,12 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tw, const GemmP
   }
   cfg.attrs = attrs;
   cfg.numAttrs = na;
-  if ((p.a_small_rows > 0) != (ta_small != nullptr)) return -19;
   return cudaLaunchKernelEx(&cfg, kern, ta, tw, ta_small ? *ta_small : ta, p) == cudaSuccess ? 0 : -4;
+}
+template <int BN, int EPI, int BUDGET_KB, bool FP4 = false, int MT = 1>
+static int launch_gemm(const ActMaps& ta, const CUtensorMap& tw, const GemmParams& p, int split, bool pdl, cudaStream_t stream) {
+  return launch_gemm<BN, EPI, BUDGET_KB, FP4, MT>(ta.full, tw, p, split, pdl, stream, 0, 0,
+                                                  p.a_small_rows > 0 ? &ta.last : nullptr);
 }
 
 }  // namespace js
@@ -1136,10 +1153,11 @@ extern "C" int js_gemm_bf16(const void* A, const void* W, void* C, const void* r
   if (epi == EPI_SWIGLU && split > 4) return -14;
   if ((epi == EPI_STORE || epi == EPI_STORE_F32) && split > bn / 32) return -14;
   if ((epi == EPI_STORE || epi == EPI_SWIGLU) && (ldc % 8)) return -15;
-  CUtensorMap ta, tw;
-  if (make_map(&ta, A, M, K, lda, BM) || make_map(&tw, W, N, K, ldw, bn)) return -16;
   GemmParams p{M, N, K, ldc, C, reinterpret_cast<const __nv_bfloat16*>(residual), part_val, part_idx, part_lse, status, trace,
                nullptr, nullptr, 0, 1, 0, nullptr, nullptr, nullptr, nullptr, nullptr};
+  ActMaps ta;
+  CUtensorMap tw;
+  if (make_act_maps(&ta, &p, A, K, lda, false) || make_map(&tw, W, N, K, ldw, bn)) return -16;
   p.m_fast = ((epi == EPI_ARGMAX || epi == EPI_TOPK) && M > BM) ? 1 : 0;
   if (deep == 3) {     // two row tiles per CTA (256 x 256 output per CTA, 192 KB pipeline): many-row GEMMs
     if (bn != 256 || split != 1) return -19;
@@ -1269,14 +1287,15 @@ extern "C" int js_gemm_nvfp4(const void* Aq, const void* sfa, const float* row_s
   if (epi == EPI_SWIGLU && split > 2) return -14;
   if ((epi == EPI_STORE || epi == EPI_SWIGLU) && (ldc % 8)) return -15;
   if (!row_scale) return -22;
-  CUtensorMap ta, tw;
-  if (make_map_u8(&ta, Aq, M, K / 2, lda_bytes, BM) || make_map_u8(&tw, Wq, N, K / 2, ldw_bytes, 128)) return -16;
   GemmParams p{};
   p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.C = C;
   p.residual = reinterpret_cast<const __nv_bfloat16*>(residual);
   p.status = status; p.world = 1;
   p.sfa = reinterpret_cast<const uint8_t*>(sfa); p.sfw = reinterpret_cast<const uint8_t*>(sfw);
   p.row_scale = row_scale; p.w_scale = w_scale;
+  ActMaps ta;
+  CUtensorMap tw;
+  if (make_act_maps(&ta, &p, Aq, K / 2, lda_bytes, true) || make_map_u8(&tw, Wq, N, K / 2, ldw_bytes, 128)) return -16;
 #define JS_CASE4(EPI_)                                                                                   \
   if (epi == EPI_)                                                                                        \
     return split > 1 ? launch_gemm<128, EPI_, 128, true>(ta, tw, p, split, pdl != 0, stream)              \
@@ -1331,11 +1350,12 @@ extern "C" int js_gemm_inproj(const void* A, const void* W, float* C, void* C2, 
   if (split < 1 || split > 4 || split > (K + BK - 1) / BK || (bn != 128 && split != 1)) return -12;
   if ((N % 128) || (n_raw % 128) || n_raw < 0 || n_raw > N || (ldc % 4) || (ldc2 % 8) || act < 0 || act > 4) return -15;
   if ((n_raw > 0 && (C == nullptr || ldc < n_raw)) || (n_raw < N && C2 == nullptr)) return -22;
-  CUtensorMap ta, tw;
-  if (make_map(&ta, A, M, K, lda, BM) || make_map(&tw, W, N, K, ldw, bn)) return -16;
   GemmParams p{};
   p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.C = C; p.status = status; p.world = 1;
   p.C2 = reinterpret_cast<__nv_bfloat16*>(C2); p.ldc2 = ldc2; p.n_raw = n_raw; p.act = act; p.act_a = act_a; p.act_b = act_b;
+  ActMaps ta;
+  CUtensorMap tw;
+  if (make_act_maps(&ta, &p, A, K, lda, false) || make_map(&tw, W, N, K, ldw, bn)) return -16;
   if (bn == 128)
     return deep == 1   ? launch_gemm<128, EPI_INPROJ, 192>(ta, tw, p, split, pdl != 0, stream)
            : deep == 2 ? launch_gemm<128, EPI_INPROJ, 128>(ta, tw, p, split, pdl != 0, stream)
@@ -1357,12 +1377,13 @@ extern "C" int js_gemm_resid32(const void* A, const void* W, float* x_out, const
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) return -11;
   if (split < 1 || split > 4 || split > (K + BK - 1) / BK || (bn != 128 && split != 1)) return -12;
   if (norm_w != nullptr && (norm_b == nullptr || h == nullptr)) return -22;
-  CUtensorMap ta, tw;
-  if (make_map(&ta, A, M, K, lda, BM) || make_map(&tw, W, N, K, ldw, bn)) return -16;
   GemmParams p{};
   p.M = M; p.N = N; p.K = K; p.ldc = ldx; p.C = x_out; p.status = status; p.world = 1;
   p.res32 = x_in; p.emb = reinterpret_cast<const __nv_bfloat16*>(emb); p.ld_emb = ld_emb;
   p.C2 = reinterpret_cast<__nv_bfloat16*>(h); p.ldc2 = ldh; p.norm_w = norm_w; p.norm_b = norm_b; p.norm_alpha = norm_alpha;
+  ActMaps ta;
+  CUtensorMap tw;
+  if (make_act_maps(&ta, &p, A, K, lda, false) || make_map(&tw, W, N, K, ldw, bn)) return -16;
   if (bn == 128)
     return deep == 1   ? launch_gemm<128, EPI_RESID32, 192>(ta, tw, p, split, pdl != 0, stream)
            : deep == 2 ? launch_gemm<128, EPI_RESID32, 128>(ta, tw, p, split, pdl != 0, stream)
@@ -1383,11 +1404,13 @@ extern "C" int js_gemm_bf16_batched(const void* A, const void* W, void* C, int M
   if ((K % 8) || (lda % 8) || (ldw % 8) || (N % 8) || (ldc % 8) || (a_batch_k % 8) || (c_batch_stride % 8)) return -10;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(C)) & 15) return -11;
   if (batch > 65535) return -12;
-  CUtensorMap ta, tw;
   const uint64_t a_cols = a_batch_k > 0 ? static_cast<uint64_t>(batch - 1) * a_batch_k + K : K;
-  if (make_map(&ta, A, M, a_cols, lda, BM) || make_map(&tw, W, static_cast<uint64_t>(batch) * N, K, ldw, 128)) return -16;
   GemmParams p{};
   p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.C = C; p.status = status; p.world = 1;
   p.batch = batch; p.a_batch_k = a_batch_k; p.c_batch_stride = c_batch_stride;
-  return launch_gemm<128, EPI_STORE, 96>(ta, tw, p, 1, pdl != 0, stream, batch, (M + BM - 1) / BM);
+  ActMaps ta;
+  CUtensorMap tw;
+  if (make_act_maps(&ta, &p, A, a_cols, lda, false) || make_map(&tw, W, static_cast<uint64_t>(batch) * N, K, ldw, 128)) return -16;
+  return launch_gemm<128, EPI_STORE, 96>(ta.full, tw, p, 1, pdl != 0, stream, batch, (M + BM - 1) / BM,
+                                         p.a_small_rows > 0 ? &ta.last : nullptr);
 }

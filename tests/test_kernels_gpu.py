@@ -82,6 +82,33 @@ def test_gemm_two_row_tiles_per_cta(ext, M):
     assert ext.pick_gemm_config(2048, 6144, 4096, ext.EPI_STORE) == (256, 1, 1)     # would be two waves of big tiles
 
 
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 127, 129, 255, 257])
+def test_gemm_last_row_tile(ext, M):
+    """The last row tile's activation box holds only the rows that are left: every entry point that takes whole matrices,
+    NaN behind the last row, row counts at the edges of the box, two row tiles per CTA with an empty second one."""
+    K, N = 320, 512
+    pad, w = rnd(M + 3, K, seed=40), rnd(N, K, scale=0.05, seed=41)
+    pad[M:] = float("nan")
+    x = pad[:M]
+    ref = x.float() @ w.float().t()
+    for kw in (dict(), dict(split=3), dict(bn=256, split=1, deep=3)):
+        assert rel_err(ext.gemm(x, w, **kw), ref) < BF16_TOL
+    act = ext.gemm(x, ext.interleave_gate_up(w[:256], w[256:]), epi=ext.EPI_SWIGLU)
+    assert rel_err(act, torch.nn.functional.silu(ref[:, :256]) * ref[:, 256:]) < BF16_TOL
+    _, best = ext.lm_head_argmax(x, w)
+    assert rel_err(best, ref.amax(-1)) < 1e-4
+    raw, act = torch.empty(M, 256, device="cuda"), torch.empty(M, 256, dtype=torch.bfloat16, device="cuda")
+    ext.gemm_inproj(x, w, raw, 256, act, False, act=ext.ACT_RELU2)
+    assert rel_err(raw, ref[:, :256]) < 1e-4 and rel_err(act, ref[:, 256:].relu() ** 2) < BF16_TOL
+    y = torch.ones(M, N, device="cuda")
+    ext.gemm_resid32(x, w, y)
+    assert rel_err(y, ref + 1) < 1e-4
+    many = torch.empty(M, 2, 256, dtype=torch.bfloat16, device="cuda")
+    ext.gemm_batched(x, w, many, 2, 256, K, 0, 256, 512)
+    assert rel_err(many.view(M, N), ref) < BF16_TOL
+    ext.check_status("cuda")
+
+
 def test_gemm_fp32_out(ext):
     x, w = rnd(64, 512, seed=6), rnd(128, 512, scale=0.05, seed=7)
     out = ext.gemm(x, w, epi=ext.EPI_STORE_F32, split=2)
