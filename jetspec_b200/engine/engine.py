@@ -255,25 +255,29 @@ class JetSpecEngine:
         self.pool.state(seq_id).length = T
         return logits, hidden
 
-    def _prefill_batch_member(self, seq_id: int, toks: torch.Tensor, taps, temperature: float):
-        """Prefill one newly admitted request of a batch.  Returns ``(first token, tap hidden | None)``.  Under
-        tensor parallelism the prompt runs through the sharded kernel path (the module forward holds full-size
+    def _prefill_admitted(self, reqs: list, taps, temperature: float) -> list:
+        """Prefill the newly admitted requests of a batch.  Returns ``[(first token, tap hidden | None)]``, in order.  Under
+        tensor parallelism the prompts run through the sharded kernel path (the module forward holds full-size
         weights and cannot address the sharded KV pool)."""
+        if not reqs:
+            return []
         if self.tp is not None and temperature > 0.0:
             raise NotImplementedError("tensor-parallel batches decode greedily")
+        prompts = [torch.tensor(r.input_ids, device=self.device) for r in reqs]
         kernel_path = self.tp is not None
         if not kernel_path and self.use_kernels and temperature <= 0.0 and self.cfg.kernel_path_ok():
             from .fast_round import FastRound
             kernel_path = FastRound.get(self)._kernel_prefill_ok()      # the same prompt path as single requests
         if kernel_path:
             from .fast_round import FastRound
-            T = int(toks.numel())
-            have = self.pool.state(seq_id).capacity if self.pool.has(seq_id) else 0
-            return FastRound.get(self)._prefill_kernels(seq_id, toks.reshape(1, -1), taps, max(T, have))
-        logits, hidden, _ = self._forward([seq_id], [toks], [0], taps=taps,
-                                          logits_rows=slice(toks.numel() - 1, toks.numel()))
-        self.pool.state(seq_id).length = toks.numel()
-        return int(sample(logits[-1], temperature)), hidden
+            return FastRound.get(self).prefill_admitted([r.seq_id for r in reqs], prompts, taps)
+        out = []
+        for r, toks in zip(reqs, prompts):
+            logits, hidden, _ = self._forward([r.seq_id], [toks], [0], taps=taps,
+                                              logits_rows=slice(toks.numel() - 1, toks.numel()))
+            self.pool.state(r.seq_id).length = toks.numel()
+            out.append((int(sample(logits[-1], temperature)), hidden))
+        return out
 
     # ------------------------------------------------------------ AR decode
     @torch.inference_mode()
@@ -536,9 +540,7 @@ class JetSpecEngine:
             if prefill_chunk:
                 self._chunked_step(sched, int(prefill_chunk), sp.temperature, results, reqs)
                 continue
-            for req in out.admitted:
-                toks = torch.tensor(req.input_ids, device=self.device)
-                first, _ = self._prefill_batch_member(req.seq_id, toks, None, sp.temperature)
+            for req, (first, _) in zip(out.admitted, self._prefill_admitted(out.admitted, None, sp.temperature)):
                 self._record_token(sched, req, first, results, reqs)
             running = [r for r in sched.running.values() if not r.is_prefill]
             if not running:
@@ -666,9 +668,8 @@ class JetSpecEngine:
             out = sched.step()
             for v in out.evicted:
                 sched.restore_sequence(v.seq_id)
-            for req in out.admitted:
+            for req, (first, hidden) in zip(out.admitted, self._prefill_admitted(out.admitted, taps, sp.temperature)):
                 toks = torch.tensor(req.input_ids, device=self.device)
-                first, hidden = self._prefill_batch_member(req.seq_id, toks, taps, sp.temperature)
                 prior = state.get(req.seq_id, {"rounds": 0, "acc": []})
                 state[req.seq_id] = {"committed": torch.cat((toks, torch.tensor([first], device=self.device))),
                                      "hidden": hidden, "rounds": prior["rounds"], "acc": prior["acc"]}

@@ -14,6 +14,7 @@ Per-sequence device state (int32 words, see ``csrc/tree_kernels.cu``):
 from __future__ import annotations
 
 import ctypes
+import itertools
 import math
 import os
 from typing import Optional
@@ -108,6 +109,10 @@ def _finish_layer_weights(out: list) -> list:
 
 
 _WIDE_GU_ROWS = 1024
+# Rows of a prefill portion: wide enough that its GEMMs are bound by the tensor cores (512-row portions took 277 us a
+# layer of Qwen3-8B's GEMMs, 4 x 277 for the rows that one 2048-row portion takes in 675), few enough that the
+# activations stay in the tens of megabytes.
+_PREFILL_ROWS = 2048
 
 
 def _gu_wide(L: dict) -> torch.Tensor:
@@ -996,13 +1001,16 @@ class FastRound:
         return n
 
     def _prefill_kernels(self, sid: int, ids: torch.Tensor, taps, total: int):
-        """Causal prefill on the kernel path in chunks (the tensor-parallel route: sharded weights,
-        fused GEMM+all-reduce).  Returns ``(first greedy token, tapped hidden (T, taps*H) or None)``."""
+        """Causal prefill on the kernel path: :meth:`_prefill_packed`, or in chunks of one prompt over several ranks
+        (sharded weights, fused GEMM+all-reduce; expert parallelism).  Returns ``(first greedy token, tapped hidden
+        (T, taps*H) or None)``."""
         pool, dev, cfg = self.eng.pool, self.device, self.cfg
         T, H = ids.shape[1], cfg.hidden_size
         pool.reserve(sid, total)
         if self.stack is not None:
             return self._prefill_ragged(sid, ids, taps)
+        if self.tp is None and self.ep is None:
+            return self._prefill_packed([sid], [ids[0]], taps)[0]
         row = pool.state(sid).row
         chunk = 512 if self.tp is None else min(512, self.tp.m_cap)
         if self.ep is not None:
@@ -1061,6 +1069,64 @@ class FastRound:
         pool.state(sid).length = T
         self._tp_graph_key = None          # eager collectives ran: a batched-verify graph must re-synchronise first
         return int(out_idx.item()), hidden
+
+    def prefill_admitted(self, sids: list, prompts: list, taps) -> list:
+        """Prompts of several requests whose pages are already theirs: ``[(first greedy token, tapped hidden or None)]``."""
+        if self.tp is None and self.ep is None and self.stack is None:
+            for sid, ids in zip(sids, prompts):
+                self.eng.pool.reserve(sid, int(ids.numel()))
+            return self._prefill_packed(sids, prompts, taps)
+        pool = self.eng.pool
+        return [self._prefill_kernels(sid, ids.reshape(1, -1), taps,
+                                      max(int(ids.numel()), pool.state(sid).capacity if pool.has(sid) else 0))
+                for sid, ids in zip(sids, prompts)]
+
+    def _prefill_packed(self, sids: list, prompts: list, taps) -> list:
+        """Causal prefill of whole prompts laid end to end and cut into portions of :data:`_PREFILL_ROWS` rows, wherever
+        the cuts fall: many short prompts share one pass over the weights, a long one takes several portions."""
+        pool, dev, cfg = self.eng.pool, self.device, self.cfg
+        H, lens = cfg.hidden_size, [int(p.numel()) for p in prompts]
+        if min(lens) < 1:
+            raise ValueError("empty prompt")
+        ends = list(itertools.accumulate(lens))
+        total = ends[-1]
+        tap_ids = list(taps) if taps else None
+        hidden = torch.empty(total, len(tap_ids) * H, dtype=torch.bfloat16, device=dev) if tap_ids else None
+        h_last = torch.empty(len(sids), H, dtype=torch.bfloat16, device=dev)
+        ids32 = torch.cat([p.reshape(-1) for p in prompts]).to(device=dev, dtype=torch.int32)
+        rows = [pool.state(sid).row for sid in sids]
+        last = cfg.num_hidden_layers - 1
+        for s0 in range(0, total, _PREFILL_ROWS):
+            n = min(_PREFILL_ROWS, total - s0)
+            parts = []                                  # (prompt, its first token here, tokens)
+            for i, (end, length) in enumerate(zip(ends, lens)):
+                lo, hi = max(s0, end - length), min(s0 + n, end)
+                if hi > lo:
+                    parts.append((i, lo - (end - length), hi - lo))
+            pos = np.concatenate([np.arange(at, at + m, dtype=np.int32) for _, at, m in parts])
+            seq = np.repeat(np.array([rows[i] for i, _, _ in parts], dtype=np.int32), [m for _, _, m in parts])
+            cu = np.cumsum([0] + [m for _, _, m in parts], dtype=np.int32)
+            meta = torch.from_numpy(np.concatenate((pos, seq, cu, np.array([rows[i] for i, _, _ in parts] + [at for _, at, _ in parts],
+                                                                           dtype=np.int32)))).to(dev)
+            pos, seq, cu_q, seq_rows, past = meta.split([n, n, len(parts) + 1, len(parts), len(parts)])
+            slots = pool.slot_map[seq.long(), pos.long()]
+            st = _Stack(self.lcfg, n, dev, pool.max_seq_len)
+            tapbuf = hidden[s0:s0 + n] if hidden is not None else None
+            X.embed(ids32[s0:s0 + n], self.embed_w, out=st.x)
+            xn = torch.empty_like(st.x)
+            decoder_layers(self.lcfg, self.layers, st, pool.k_pool, pool.v_pool, pool.slot_map, seq_rows, cu_q, past,
+                           pos, slots, None, True, self.freq, taps=tapbuf, tap_ids=tap_ids, pdl=False,
+                           final_norm=(self.final_norm, xn))
+            for j, t in enumerate(tap_ids or ()):
+                if t == last:
+                    tapbuf[:, j * H:(j + 1) * H] = xn
+            done = [(i, int(c) - 1) for (i, at, m), c in zip(parts, cu[1:]) if at + m == lens[i]]
+            if done:
+                h_last[[i for i, _ in done]] = xn[[r for _, r in done]]
+        first, _ = X.lm_head_argmax(h_last, self.lm_head_w)
+        for sid, n in zip(sids, lens):
+            pool.state(sid).length = n
+        return [(int(t), hidden[end - n:end] if hidden is not None else None) for t, end, n in zip(first.tolist(), ends, lens)]
 
     def _prefill_ragged(self, sid: int, ids: torch.Tensor, taps, chunk: int = 2048):
         """Prompt of one sequence through :meth:`ragged_forward` in portions of ``chunk`` tokens; same results as

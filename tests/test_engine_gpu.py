@@ -427,3 +427,28 @@ def test_batched_graph_verify_is_lossless_and_matches_the_eager_batch(engine, sm
         agree, short = teacher_forced_agreement(small, p, o["token_ids"])
         assert agree > 0.85 and short < 0.05
     cuda_ext.check_status("cuda")
+
+
+@pytest.mark.parametrize("portion", [1, 50, 64, 2048])
+def test_prompts_prefilled_together(engine, monkeypatch, portion):
+    """Prompts laid end to end and cut into portions anywhere: first tokens, tapped hidden states and the pool's lengths equal
+    those of each prompt alone on the module path (bf16 tolerance)."""
+    from jetspec_b200.engine import fast_round
+    monkeypatch.setattr(fast_round, "_PREFILL_ROWS", portion)
+    g = torch.Generator().manual_seed(5)
+    lens = [1, 70, 33, 64] if portion > 1 else [1, 3]
+    prompts = [torch.randint(0, 4096, (n,), generator=g).cuda() for n in lens]
+    taps = [1, 3]
+    engine._ensure_pool(1024, seqs=8)
+    fast, sids = fast_round.FastRound.get(engine), [engine._new_seq_id() for _ in range(2 * len(lens))]
+    try:
+        with torch.inference_mode():
+            got = fast.prefill_admitted(sids[:len(lens)], prompts, taps)
+            for sid, ref_sid, p, (first, hidden) in zip(sids, sids[len(lens):], prompts, got):
+                logits, want = engine._prefill(ref_sid, p, taps=taps)
+                assert engine.pool.state(sid).length == p.numel() and hidden.shape == want.shape
+                assert float((hidden.float() - want.float()).norm() / want.float().norm()) < 2e-2
+                assert float(logits[-1].max() - logits[-1][first]) <= 0.02 * float(logits[-1].abs().max())
+    finally:
+        for sid in sids:
+            engine.pool.free(sid)
