@@ -29,93 +29,12 @@
 // Epilogues: plain store (+ residual), SwiGLU (the tile holds BN/2 gate and BN/2 up columns
 // of the same outputs), per-tile argmax partials (LM head), per-tile top-8 + log-sum-exp
 // partials (draft head logits).
-#include "common.cuh"
-
-#include <math.h>
+#include "gemm_common.cuh"
 
 namespace js {
 
-constexpr int BM = 128;
-constexpr int BK = 64;          // 64 bf16 = one 128-byte swizzle row
-constexpr int UMMA_K = 16;
 constexpr int kGemmThreads = 192;
 constexpr int kTopK = 8;
-
-enum GemmEpi : int { EPI_STORE = 0, EPI_SWIGLU = 1, EPI_ARGMAX = 2, EPI_TOPK = 3, EPI_STORE_F32 = 4, EPI_ALLREDUCE = 5, EPI_EP_COMBINE = 6,
-                    EPI_INPROJ = 7, EPI_RELU2 = 8, EPI_RESID32 = 9 };
-enum GemmAct : int { ACT_GELU_GLU = 0, ACT_RELU2 = 1, ACT_NONE = 2, ACT_GELU_ERF = 3, ACT_XIELU = 4 };
-
-struct GemmParams {
-  int M, N, K;
-  int ldc;                      // elements
-  void* C;                      // bf16 (or fp32 for EPI_STORE_F32) output
-  const __nv_bfloat16* residual;  // optional, same shape/ld as C (may alias C)
-  float* part_val;              // ARGMAX: [M, n_tiles] ; TOPK: [M, n_tiles, 8] values
-  int* part_idx;                // ARGMAX: [M, n_tiles] ; TOPK: [M, n_tiles, 8] indices
-  float* part_lse;              // TOPK: [M, n_tiles, 2] (running max, sum of exp)
-  int* status;
-  unsigned long long* trace;    // optional: 8 phase timestamps (ns) written by CTA (0,0,0)
-  // EPI_ALLREDUCE (tensor-parallel row-parallel GEMM): every rank's receive buffer and flag array
-  __nv_bfloat16* const* peer_recv;  // [world] -> (world, m_cap, N) bf16 on that rank
-  int* const* peer_flags;           // [world] -> one counter per CTA of this grid on that rank
-  int rank, world, m_cap;
-  // grouped mode (MoE experts): blockIdx.z is the expert; its rows are group_off[e] .. group_off[e+1]
-  // of A and C, its weights are rows e*N .. (e+1)*N of W.  No K split in this mode.
-  const int* group_off;
-  // EPI_EP_COMBINE (expert-parallel down projection): row r of the sorted rows belongs to
-  // (token, choice) pair row_pair[r] with routing weight row_weight[r]; the weighted output row is
-  // stored into every rank's pair buffer (n_pairs, N) and a per-rank counter is bumped per CTA.
-  const int* row_pair;
-  const float* row_weight;
-  __nv_bfloat16* const* peer_pairs;
-  int* const* peer_cnt;
-  // EPI_EP_COMBINE with token-sharded dispatch: row r of this rank's receive slab came from rank row_meta[r].x
-  // as that rank's (token, choice) pair row_meta[r].y; the weighted output row returns to that rank only, as
-  // flagged 8-byte cells {two bf16 values, 1} that the owner's finishing kernel polls (no counters)
-  const int2* row_meta;
-  // NVFP4 mode: block scales of A and W in 512-byte tiles, per-row scale of A, per-tensor scale of W
-  const uint8_t* sfa;
-  const uint8_t* sfw;
-  const float* row_scale;
-  float w_scale;
-  // EPI_ALLREDUCE: only push the partial tile and bump the flags; a finishing kernel reduces (no wait in this kernel)
-  int ar_push_only;
-  // Tile order: 0 = column tiles fastest (consecutive CTAs share the activation tile), 1 = row tiles fastest
-  // (consecutive CTAs share the WEIGHT tile: for a vocabulary matrix larger than L2 and many row tiles, each
-  // weight tile then comes from HBM once instead of once per row tile)
-  int m_fast;
-  // A row tile with at most this many rows left loads its activations through the second tensor map, whose box holds
-  // only that many rows (0 = always the 128-row box); the accumulator rows beyond the box read stale shared memory
-  // and are never stored.  Grouped mode: with ~8 rows per expert (MoE decode) a 128-row box would make the
-  // activations half of every stage's bytes although almost none of its rows are used.  Otherwise it is M % 128, so
-  // that the last row tile's box ends with the matrix: a box that lies mostly past the end is slow, because every CTA
-  // waits for its zero fill (4096 x 24576 weights at 1 row, 128-row box against 1-row box: 69.1 against 40.2 us per
-  // launch, 4096 x 6144 at 8 rows 24.2 against 15.5, 4096 x 151936 at 1 row 276 against 203; equal from 16 rows on).
-  int a_small_rows;
-  // EPI_INPROJ (fused input projections of a parallel block): columns below n_raw (a multiple of 128) are stored as
-  // fp32 to C; the rest pass through `act` and go to C2 as bf16.  ACT_GELU_GLU: every 128 weight rows hold 64 gate rows
-  // and the 64 up rows of the same outputs; ACT_RELU2: relu(.)^2 of each column; ACT_GELU_ERF: exact gelu of each
-  // column; ACT_XIELU: act_a z^2 + z / 2 for z > 0, act_b (e^z - 1 - z) + z / 2 below; ACT_NONE: as it is.
-  __nv_bfloat16* C2;
-  int ldc2;
-  int n_raw;
-  int act;
-  float act_a, act_b;
-  // EPI_RESID32: C (fp32) = res32 + A W^T (+ emb); with norm_w, C2 = bf16(tanh(norm_alpha C) norm_w + norm_b), the
-  // next layer's Dynamic Tanh.  res32 may be C.
-  const float* res32;
-  const __nv_bfloat16* emb;
-  int ld_emb;
-  const float* norm_w;
-  const float* norm_b;
-  float norm_alpha;
-  // Batched mode: blockIdx.z is the batch element; its K columns of A start at z * a_batch_k, its weights are rows
-  // z*N .. (z+1)*N of W, its output starts at C + z * c_batch_stride.  A box that reaches past the element's own K
-  // columns meets zero-filled weights.  No K split in this mode.
-  int batch;
-  int a_batch_k;
-  long long c_batch_stride;
-};
 
 JS_DEVICE void red_release_sys_add(int* addr, int v) {
   asm volatile("red.release.sys.global.add.s32 [%0], %1;" ::"l"(addr), "r"(v) : "memory");
@@ -256,122 +175,130 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   // to finish before touching our output.
   pdl_launch_dependents();
 
+  // The producing and the issuing warp run their loops with all lanes, stage and phase counted up rather than divided out,
+  // and one elected lane issues.  Under `if (lane == 0)` every operand of the issue sat in per-thread registers, and a
+  // 64-wide k-block cost 0.29 us of that one thread whatever the tile: 512 x 4096 x 12288 took 63.4 us on 128 x 128 tiles
+  // (52.3 this way) and 118 us on 64-column tiles (89).
   if (warp == 0) {
-    if (lane == 0) {
-      JS_TRACE(1);   // setup done, first TMA about to issue
-      // Weights do not depend on the previous kernel: start streaming them before waiting on it.
-      const int pre = nkb < kStages ? nkb : kStages;
-      // FP4: scale tiles of k-block kb are 4 consecutive 512-byte tiles of this operand's row tile
-      const size_t sf_row = static_cast<size_t>(p.K / 64) * 512;
-      auto load_sfw = [&](int s, int kb) {
-        if constexpr (FP4)
-          bulk_load_1d(smem + s * S::kStage + S::kStageA + S::kStageW + 2048,
-                       p.sfw + static_cast<size_t>(wn0 / 128) * sf_row + static_cast<size_t>(kb) * 2048, 2048, &full_bar[s]);
-      };
-      auto load_sfa = [&](int s, int kb) {
-        if constexpr (FP4)
-          bulk_load_1d(smem + s * S::kStage + S::kStageA + S::kStageW,
-                       p.sfa + static_cast<size_t>(m0 / 128) * sf_row + static_cast<size_t>(kb) * 2048, 2048, &full_bar[s]);
-      };
-      // bytes a stage receives: the activation box shrinks for a row tile with few rows left (grouped mode)
-      auto box_rows = [&](int m) {       // rows of the activation box of the row tile at m (0: no rows left, MT == 2 only)
-        if (MT == 2 && m >= m_end) return 0;
-        return p.a_small_rows > 0 && m_end - m <= p.a_small_rows ? p.a_small_rows : BM;
-      };
-      auto stage_bytes = [&](int m_tile) {
-        int rows = box_rows(m_tile);
-        if constexpr (MT == 2) rows += box_rows(m_tile + BM);
-        return static_cast<uint32_t>(S::kStage - S::kStageA + rows * BK * 2);
-      };
-      auto load_a = [&](int s, int x, int m_tile) {
+    if (lane == 0) JS_TRACE(1);   // setup done, first TMA about to issue
+    // Weights do not depend on the previous kernel: start streaming them before waiting on it.
+    const int pre = nkb < kStages ? nkb : kStages;
+    // FP4: scale tiles of k-block kb are 4 consecutive 512-byte tiles of this operand's row tile
+    const size_t sf_row = static_cast<size_t>(p.K / 64) * 512;
+    auto load_w = [&](int s, int kb) {
+      tma_load_2d(smem + s * S::kStage + S::kStageA, &tmW, &full_bar[s], kb * kXStep, wn0);
+      if constexpr (FP4)
+        bulk_load_1d(smem + s * S::kStage + S::kStageA + S::kStageW + 2048,
+                     p.sfw + static_cast<size_t>(wn0 / 128) * sf_row + static_cast<size_t>(kb) * 2048, 2048, &full_bar[s]);
+    };
+    // bytes a stage receives: the activation box shrinks for a row tile with few rows left
+    auto box_rows = [&](int m) {       // rows of the activation box of the row tile at m (0: no rows left, MT == 2 only)
+      if (MT == 2 && m >= m_end) return 0;
+      return p.a_small_rows > 0 && m_end - m <= p.a_small_rows ? p.a_small_rows : BM;
+    };
+    auto stage_bytes = [&](int m_tile) {
+      int rows = box_rows(m_tile);
+      if constexpr (MT == 2) rows += box_rows(m_tile + BM);
+      return static_cast<uint32_t>(S::kStage - S::kStageA + rows * BK * 2);
+    };
+    auto load_a = [&](int s, int kb, int m_tile) {
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-          const int rows = box_rows(m_tile + mt * BM);
-          if (rows > 0)
-            tma_load_2d(smem + s * S::kStage + mt * (BM * BK * 2), rows == BM ? &tmA : &tmA2, &full_bar[s], x, m_tile + mt * BM);
-        }
-      };
-      const uint32_t bytes0 = stage_bytes(m0);
+      for (int mt = 0; mt < MT; ++mt) {
+        const int rows = box_rows(m_tile + mt * BM);
+        uint8_t* dst = smem + s * S::kStage + mt * (BM * BK * 2);
+        const int x = ax0 + kb * kXStep, y = m_tile + mt * BM;
+        if (rows == BM) tma_load_2d(dst, &tmA, &full_bar[s], x, y);
+        else if (rows > 0) tma_load_2d(dst, &tmA2, &full_bar[s], x, y);
+      }
+      if constexpr (FP4)
+        bulk_load_1d(smem + s * S::kStage + S::kStageA + S::kStageW,
+                     p.sfa + static_cast<size_t>(m0 / 128) * sf_row + static_cast<size_t>(kb) * 2048, 2048, &full_bar[s]);
+    };
+    const uint32_t bytes0 = stage_bytes(m0);
+    if (elect_one()) {
       for (int i = 0; i < pre; ++i) {
         mbar_expect_tx(&full_bar[i], bytes0);
-        tma_load_2d(smem + i * S::kStage + S::kStageA, &tmW, &full_bar[i], (kb_begin + i) * kXStep, wn0);
-        load_sfw(i, kb_begin + i);
+        load_w(i, kb_begin + i);
       }
-      pdl_wait();
-      for (int i = 0; i < pre; ++i) {
-        load_a(i, ax0 + (kb_begin + i) * kXStep, m0);
-        load_sfa(i, kb_begin + i);
-      }
-      bool p_ok = true;
-      for (int tj = 0; tj < n_tiles_cta && p_ok; ++tj) {
-        const int m_tile = m_first + tj * tile_step;
-        const uint32_t bytes = stage_bytes(m_tile);
-        for (int i = (tj == 0 ? pre : 0); i < nkb; ++i) {
-          const int g = tj * nkb + i;              // running k-block count of this CTA
-          const int s = g % kStages;
-          if (g >= kStages) {
-            const uint32_t ph = (g / kStages) & 1;
-            if (!mbar_wait(&empty_bar[s], ph ^ 1, p.status, kTimeoutEmpty)) { p_ok = false; break; }
-          }
+    }
+    __syncwarp();
+    pdl_wait();
+    if (elect_one()) {
+      for (int i = 0; i < pre; ++i) load_a(i, kb_begin + i, m0);
+    }
+    __syncwarp();
+    bool p_ok = true;
+    int s = pre == kStages ? 0 : pre;
+    uint32_t phase = pre == kStages ? 0 : 1;       // of the empty barriers: the first round finds every stage free
+    for (int tj = 0; tj < n_tiles_cta && p_ok; ++tj) {
+      const int m_tile = m_first + tj * tile_step;
+      const uint32_t bytes = stage_bytes(m_tile);
+      for (int i = (tj == 0 ? pre : 0); i < nkb; ++i) {
+        p_ok = mbar_wait(&empty_bar[s], phase, p.status, kTimeoutEmpty);
+        if (!p_ok) break;
+        if (elect_one()) {
           mbar_expect_tx(&full_bar[s], bytes);
-          tma_load_2d(smem + s * S::kStage + S::kStageA, &tmW, &full_bar[s], (kb_begin + i) * kXStep, wn0);
-          load_a(s, ax0 + (kb_begin + i) * kXStep, m_tile);
-          load_sfw(s, kb_begin + i);
-          load_sfa(s, kb_begin + i);
+          load_w(s, kb_begin + i);
+          load_a(s, kb_begin + i, m_tile);
         }
+        __syncwarp();
+        if (++s == kStages) { s = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = FP4 ? umma_idesc_nvfp4(BM, BN) : umma_idesc_bf16(BM, BN);
-      bool ok = true;
-      for (int tj = 0; tj < n_tiles_cta && ok; ++tj) {
+    constexpr uint32_t idesc = FP4 ? umma_idesc_nvfp4(BM, BN) : umma_idesc_bf16(BM, BN);
+    const uint64_t desc0 = umma_desc_sw128(smem_u32(smem));
+    const uint64_t sf_desc0 = umma_desc_sf(smem_u32(smem) + S::kStageA + S::kStageW);
+    bool ok = true;
+    int s = 0;
+    uint32_t phase = 0;
+    for (int tj = 0; tj < n_tiles_cta && ok; ++tj) {
       if (tj > 0) {                 // the epilogue must have read the previous row tile out of tensor memory
         ok = mbar_wait(tmem_free, (tj - 1) & 1, p.status, kTimeoutAccum);
         if (!ok) break;
         tc_fence_after();
       }
+      uint32_t more = 0;            // 0: the accumulator starts anew
       for (int i = 0; i < nkb && ok; ++i) {
-        const int g = tj * nkb + i;
-        const int s = g % kStages;
-        const uint32_t ph = (g / kStages) & 1;
-        ok = mbar_wait(&full_bar[s], ph, p.status, kTimeoutFull);
+        ok = mbar_wait(&full_bar[s], phase, p.status, kTimeoutFull);
         if (!ok) break;
-        if (g == 0) JS_TRACE(2);   // first stage landed
+        if (lane == 0 && tj == 0 && i == 0) JS_TRACE(2);   // first stage landed
         tc_fence_after();
-        const uint64_t a_desc = umma_desc_sw128(smem_u32(smem + s * S::kStage));
-        const uint64_t b_desc = umma_desc_sw128(smem_u32(smem + s * S::kStage + S::kStageA));
-        if constexpr (FP4) {
-          // scale tiles: shared memory -> tensor memory (4 columns per 128 rows x 4 blocks), then
-          // four K=64 MMAs, each reading its own 4+4 scale columns
-          const uint32_t sf_smem = smem_u32(smem + s * S::kStage + S::kStageA + S::kStageW);
-          const uint32_t sf_tmem = tmem_base + 128 + s * 32;
+        if (elect_one()) {
+          const uint64_t a_desc = desc0 + static_cast<uint64_t>(s * (S::kStage >> 4));
+          const uint64_t b_desc = a_desc + (S::kStageA >> 4);
+          if constexpr (FP4) {
+            // scale tiles: shared memory -> tensor memory (4 columns per 128 rows x 4 blocks), then
+            // four K=64 MMAs, each reading its own 4+4 scale columns
+            const uint64_t sf_desc = sf_desc0 + static_cast<uint64_t>(s * (S::kStage >> 4));
+            const uint32_t sf_tmem = tmem_base + 128 + s * 32;
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            tmem_cp_32x128b_warpx4(sf_tmem + 4 * k, umma_desc_sf(sf_smem + 512 * k));
-            tmem_cp_32x128b_warpx4(sf_tmem + 16 + 4 * k, umma_desc_sf(sf_smem + 2048 + 512 * k));
-          }
+            for (int k = 0; k < 4; ++k) {
+              tmem_cp_32x128b_warpx4(sf_tmem + 4 * k, sf_desc + 32 * k);
+              tmem_cp_32x128b_warpx4(sf_tmem + 16 + 4 * k, sf_desc + 128 + 32 * k);
+            }
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            // advancing K by 64 e2m1 = 32 bytes inside the swizzle row = +2 in 16-byte units
-            umma_nvfp4(tmem_base, a_desc + 2 * k, b_desc + 2 * k, idesc, sf_tmem + 4 * k, sf_tmem + 16 + 4 * k,
-                       (i | k) != 0 ? 1u : 0u);
-          }
-        } else {
+            for (int k = 0; k < 4; ++k) {
+              // advancing K by 64 e2m1 = 32 bytes inside the swizzle row = +2 in 16-byte units
+              umma_nvfp4(tmem_base, a_desc + 2 * k, b_desc + 2 * k, idesc, sf_tmem + 4 * k, sf_tmem + 16 + 4 * k, k == 0 ? more : 1u);
+            }
+          } else {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            // advancing K by 16 elements = 32 bytes inside the swizzle row = +2 in 16-byte units
-            umma_f16(tmem_base, a_desc + 2 * k, b_desc + 2 * k, idesc, (i | k) != 0 ? 1u : 0u);
-            if constexpr (MT == 2) {     // second row tile: its own A rows and accumulator, the same weight stage
-              const uint64_t a2_desc = umma_desc_sw128(smem_u32(smem + s * S::kStage + BM * BK * 2));
-              umma_f16(tmem_base + BN, a2_desc + 2 * k, b_desc + 2 * k, idesc, (i | k) != 0 ? 1u : 0u);
+            for (int k = 0; k < BK / UMMA_K; ++k) {
+              // advancing K by 16 elements = 32 bytes inside the swizzle row = +2 in 16-byte units
+              umma_f16(tmem_base, a_desc + 2 * k, b_desc + 2 * k, idesc, k == 0 ? more : 1u);
+              if constexpr (MT == 2)       // second row tile: its own A rows and accumulator, the same weight stage
+                umma_f16(tmem_base + BN, a_desc + (BM * BK * 2 >> 4) + 2 * k, b_desc + 2 * k, idesc, k == 0 ? more : 1u);
             }
           }
+          umma_commit(&empty_bar[s]);   // frees the stage once these MMAs have read it
         }
-        umma_commit(&empty_bar[s]);   // frees the stage once these MMAs have read it
+        __syncwarp();
+        more = 1;
+        if (++s == kStages) { s = 0; phase ^= 1; }
       }
-      umma_commit(accum_bar);         // accumulator complete (also releases the epilogue on error)
-      }
+      if (elect_one()) umma_commit(accum_bar);         // accumulator complete (also releases the epilogue on error)
+      __syncwarp();
     }
   }
 
@@ -657,112 +584,20 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
     } else if constexpr (EPI == EPI_INPROJ) {
       // every 128-column block is handled as two 64-column halves (gate | up, or simply neighbours)
-      auto store_bf16 = [&](__nv_bfloat16* out, const float* v) {
-#pragma unroll
-        for (int j = 0; j < 32; j += 8) {
-          uint4 ov;
-          __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&ov);
-#pragma unroll
-          for (int t = 0; t < 4; ++t) o2[t] = __floats2bfloat162_rn(v[j + 2 * t], v[j + 2 * t + 1]);
-          *reinterpret_cast<uint4*>(out + j) = ov;
-        }
-      };
       for (int c0 = z * 32; c0 < BN / 2; c0 += split * 32) {
         const int blk = c0 >> 6, cb = c0 & 63;
         const int nb = n0 + blk * 128;
         float g[32], u[32];
         load_chunk(blk * 128 + cb, g);
         load_chunk(blk * 128 + 64 + cb, u);
-        if (grow >= m_end || nb >= p.N) continue;
-        if (nb < p.n_raw) {
-          float* out = reinterpret_cast<float*>(p.C) + static_cast<size_t>(grow) * p.ldc + nb + cb;
-#pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            *reinterpret_cast<float4*>(out + j) = make_float4(g[j], g[j + 1], g[j + 2], g[j + 3]);
-            *reinterpret_cast<float4*>(out + 64 + j) = make_float4(u[j], u[j + 1], u[j + 2], u[j + 3]);
-          }
-          continue;
-        }
-        __nv_bfloat16* out2 = p.C2 + static_cast<size_t>(grow) * p.ldc2;
-        if (p.act == ACT_GELU_GLU) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float a = g[j];
-            g[j] = 0.5f * a * (1.f + tanhf(0.7978845608028654f * (a + 0.044715f * a * a * a))) * u[j];   // sqrt(2 / pi)
-          }
-          store_bf16(out2 + (nb - p.n_raw) / 2 + cb, g);
-        } else {
-          if (p.act == ACT_RELU2) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              g[j] = fmaxf(g[j], 0.f);
-              g[j] *= g[j];
-              u[j] = fmaxf(u[j], 0.f);
-              u[j] *= u[j];
-            }
-          } else if (p.act == ACT_GELU_ERF) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              g[j] = 0.5f * g[j] * (1.f + erff(g[j] * 0.7071067811865476f));      // 1 / sqrt(2)
-              u[j] = 0.5f * u[j] * (1.f + erff(u[j] * 0.7071067811865476f));
-            }
-          } else if (p.act == ACT_XIELU) {
-            auto xielu = [&](float z) { return 0.5f * z + (z > 0.f ? p.act_a * z * z : p.act_b * (__expf(z) - 1.f - z)); };
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              g[j] = xielu(g[j]);
-              u[j] = xielu(u[j]);
-            }
-          }
-          store_bf16(out2 + nb - p.n_raw + cb, g);
-          store_bf16(out2 + nb - p.n_raw + 64 + cb, u);
-        }
+        if (grow < m_end && nb < p.N) epi_inproj_halves(p, grow, nb, cb, g, u);
       }
     } else if constexpr (EPI == EPI_RESID32) {
       for (int c0 = z * 32; c0 < BN; c0 += split * 32) {
         float v[32];
         load_chunk(c0, v);
         const int gc = n0 + c0;
-        if (grow >= m_end || gc >= p.N) continue;
-        float* out = reinterpret_cast<float*>(p.C) + static_cast<size_t>(grow) * p.ldc + gc;
-        const float* res = p.res32 + static_cast<size_t>(grow) * p.ldc + gc;
-        const __nv_bfloat16* emb = p.emb ? p.emb + static_cast<size_t>(grow) * p.ld_emb + gc : nullptr;
-#pragma unroll
-        for (int j = 0; j < 32; j += 8) {
-          if (gc + j >= p.N) break;
-#pragma unroll
-          for (int t = 0; t < 8; t += 4) {
-            const float4 rv = *reinterpret_cast<const float4*>(res + j + t);
-            v[j + t] += rv.x;
-            v[j + t + 1] += rv.y;
-            v[j + t + 2] += rv.z;
-            v[j + t + 3] += rv.w;
-          }
-          if (emb != nullptr) {
-            const uint4 ev = *reinterpret_cast<const uint4*>(emb + j);
-            const __nv_bfloat162* e2 = reinterpret_cast<const __nv_bfloat162*>(&ev);
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-              const float2 f = __bfloat1622float2(e2[t]);
-              v[j + 2 * t] += f.x;
-              v[j + 2 * t + 1] += f.y;
-            }
-          }
-          *reinterpret_cast<float4*>(out + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-          *reinterpret_cast<float4*>(out + j + 4) = make_float4(v[j + 4], v[j + 5], v[j + 6], v[j + 7]);
-          if (p.norm_w != nullptr) {
-            uint4 ov;
-            __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&ov);
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-              const float2 w2 = __ldg(reinterpret_cast<const float2*>(p.norm_w + gc + j + 2 * t));
-              const float2 b2 = __ldg(reinterpret_cast<const float2*>(p.norm_b + gc + j + 2 * t));
-              o2[t] = __floats2bfloat162_rn(tanhf(p.norm_alpha * v[j + 2 * t]) * w2.x + b2.x,
-                                            tanhf(p.norm_alpha * v[j + 2 * t + 1]) * w2.y + b2.y);
-            }
-            *reinterpret_cast<uint4*>(p.C2 + static_cast<size_t>(grow) * p.ldc2 + gc + j) = ov;
-          }
-        }
+        if (grow < m_end && gc < p.N) epi_resid32_chunk(p, grow, gc, v);
       }
     } else if constexpr (EPI == EPI_STORE || EPI == EPI_STORE_F32 || EPI == EPI_RELU2) {
       // 32-column chunks are dealt round-robin to the CTAs of the K-split cluster
@@ -770,44 +605,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         float v[32];
         load_chunk(c0, v);
         const int gc = n0 + c0;
-        if (grow < m_end && gc < p.N) {
-          if constexpr (EPI == EPI_STORE_F32) {
-            float* out = reinterpret_cast<float*>(p.C) + static_cast<size_t>(grow) * p.ldc + gc;
-#pragma unroll
-            for (int j = 0; j < 32; j += 4)
-              if (gc + j < p.N) *reinterpret_cast<float4*>(out + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-          } else {
-            __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<size_t>(grow) * p.ldc + gc +
-                                 p.c_batch_stride * expert;
-            const __nv_bfloat16* res = p.residual ? p.residual + static_cast<size_t>(grow) * p.ldc + gc : nullptr;
-            if constexpr (EPI == EPI_RELU2) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                v[j] = fmaxf(v[j], 0.f);
-                v[j] *= v[j];
-              }
-            }
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              if (gc + j >= p.N) break;
-              if (res) {
-                uint4 rv = *reinterpret_cast<const uint4*>(res + j);
-                const __nv_bfloat162* r2 = reinterpret_cast<const __nv_bfloat162*>(&rv);
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                  float2 f = __bfloat1622float2(r2[t]);
-                  v[j + 2 * t] += f.x;
-                  v[j + 2 * t + 1] += f.y;
-                }
-              }
-              uint4 ov;
-              __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&ov);
-#pragma unroll
-              for (int t = 0; t < 4; ++t) o2[t] = __floats2bfloat162_rn(v[j + 2 * t], v[j + 2 * t + 1]);
-              *reinterpret_cast<uint4*>(out + j) = ov;
-            }
-          }
-        }
+        if (grow < m_end && gc < p.N) epi_store_chunk<EPI>(p, grow, gc, v, p.c_batch_stride * expert);
       }
     } else if constexpr (EPI == EPI_SWIGLU) {
       constexpr int HALF = BN / 2;
@@ -816,20 +614,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         load_chunk(c0, g);
         load_chunk(HALF + c0, u);
         const int gc = n0 / 2 + c0;              // output column
-        if (grow < m_end && gc < p.N / 2) {
-          __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<size_t>(grow) * p.ldc + gc;
-#pragma unroll
-          for (int j = 0; j < 32; j += 8) {
-            uint4 ov;
-            __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&ov);
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-              const float a = g[j + 2 * t], b = g[j + 2 * t + 1];
-              o2[t] = __floats2bfloat162_rn(a / (1.f + __expf(-a)) * u[j + 2 * t], b / (1.f + __expf(-b)) * u[j + 2 * t + 1]);
-            }
-            *reinterpret_cast<uint4*>(out + j) = ov;
-          }
-        }
+        if (grow < m_end && gc < p.N / 2) epi_swiglu_chunk(p, grow, gc, g, u);
       }
     } else if constexpr (EPI == EPI_ARGMAX) {
       float best = -INFINITY;
@@ -1036,59 +821,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
 // ---------------------------------------------------------------------------- host side
 constexpr int kGroupedSmallRows = 32;     // rows of the small activation box of grouped launches (GemmParams::a_small_rows)
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn get_encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (fn == nullptr) {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) == cudaSuccess &&
-        qres == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(ptr);
-  }
-  return fn;
-}
-
-// 2-D bf16 row-major tensor [rows, cols] with leading dimension ld (elements), box = [box_rows, 64]
-static int make_map(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
-  EncodeTiledFn fn = get_encode_fn();
-  if (!fn) return -1;
-  cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {ld * 2};
-  cuuint32_t box[2] = {BK, box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 0 : -2;
-}
-
-// 2-D packed-e2m1 matrix seen as bytes: [rows, row_bytes] with leading dimension ld_bytes, box = [box_rows, 128 bytes]
-static int make_map_u8(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t row_bytes, uint64_t ld_bytes, uint32_t box_rows) {
-  EncodeTiledFn fn = get_encode_fn();
-  if (!fn) return -1;
-  cuuint64_t dims[2] = {row_bytes, rows};
-  cuuint64_t strides[1] = {ld_bytes};
-  cuuint32_t box[2] = {128, box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 0 : -2;
-}
-
-// Activation maps of a launch over M rows: full 128-row boxes, and the box of the last row tile (GemmParams::a_small_rows)
-struct ActMaps { CUtensorMap full, last; };
-static int make_act_maps(ActMaps* m, GemmParams* p, const void* A, uint64_t cols, uint64_t ld, bool u8) {
-  auto make = u8 ? make_map_u8 : make_map;
-  p->a_small_rows = p->M % BM;
-  if (make(&m->full, A, p->M, cols, ld, BM)) return -1;
-  return p->a_small_rows > 0 ? make(&m->last, A, p->M, cols, ld, p->a_small_rows) : 0;
-}
-
 template <int BN, int EPI, int BUDGET_KB, bool FP4 = false, int MT = 1>
 static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tw, const GemmParams& p, int split, bool pdl,
                        cudaStream_t stream, int groups = 0, int group_m_tiles = 0, const CUtensorMap* ta_small = nullptr) {
