@@ -108,7 +108,6 @@ def _finish_layer_weights(out: list) -> list:
     return out
 
 
-_WIDE_GU_ROWS = 1024
 # Rows of a prefill portion: wide enough that its GEMMs are bound by the tensor cores (512-row portions took 277 us a
 # layer of Qwen3-8B's GEMMs, 4 x 277 for the rows that one 2048-row portion takes in 675), few enough that the
 # activations stay in the tens of megabytes.
@@ -283,12 +282,7 @@ def decoder_layers(cfg, layers, st: _Stack, k_pools, v_pools, slot_map, seq_rows
             continue
         if pf is not None:
             pf.ahead(L["down"])
-        if st.T >= _WIDE_GU_ROWS and tp is None:
-            # many row tiles (batched verify, long prefill): compute bound, 128x256 tiles measured 24 % faster at
-            # 2048 rows (519 -> 396 us); the 256-interleaved copy of the weight is made on first use
-            X.gemm(st.h, _gu_wide(L), out=st.act, epi=X.EPI_SWIGLU, bn=256, split=1, deep=0, pdl=pdl)
-        else:
-            X.gemm(st.h, L["gu"], out=st.act, epi=X.EPI_SWIGLU, bn=L.get("gu_bn"), pdl=pdl)
+        X.gemm(st.h, L["gu"], out=st.act, epi=X.EPI_SWIGLU, bn=L.get("gu_bn"), pdl=pdl)
         if pf is not None:
             nxt = layers[li + 1]["qkv"] if li != last else then_prefetch
             if nxt is not None:

@@ -284,19 +284,48 @@ def pick_gemm_config(M: int, N: int, K: int, epi: int, bn: Optional[int] = None)
     return bn, 1, (1 if tiles <= SM_COUNT or _DEEP else 0)
 
 
+SM_PAIRS = SM_COUNT // 2
+
+
+def pick_pair_tile(M: int, N: int, K: int, interleave: int = 128) -> int:
+    """Width of the 256-row tiles of the CTA-pair GEMM, or 0 where single CTAs are as fast: the least number of k-blocks
+    that pass one after the other, weighed with what a 64-wide k-block takes.
+
+    Measured slopes (microseconds a k-block, 4096 x 4096 and 4096 x 12288 weights at 256 and 512 rows): pairs 0.285 on 256
+    columns (the tensor pipe) and 0.19 on 128 columns (the L2-to-SM path); single CTAs 0.235 on 128 x 128 tiles, which can
+    split K.  At 2048 rows (microseconds, single CTAs against pairs): 4096 x 6144 91.6 / 78.8, 4096 x 24576 388 / 269,
+    4096 x 151936 2037 / 1542; at 512 rows 4096 x 24576 124 / 79, 12288 x 4096 70 / 47; but at 256 rows 12288 x 4096 with
+    K split in two 30.6 / 42."""
+    if M <= 128 or interleave not in (128, 256):
+        return 0
+    rows, single = (M + 255) // 256, (M + 127) // 128 * ((N + 127) // 128)
+    passes = lambda tiles: (tiles + SM_PAIRS - 1) // SM_PAIRS
+    wide, narrow = 0.285 * passes(rows * ((N + 255) // 256)), 0.19 * passes(rows * ((N + 127) // 128))
+    if single <= SM_COUNT and 0.235 / pick_gemm_config(128, single * 128, K, EPI_STORE, 128)[1] <= min(wide, narrow):
+        return 0
+    return 128 if narrow < wide and interleave == 128 else 256
+
+
 def gemm(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None,
          residual: Optional[torch.Tensor] = None, epi: int = EPI_STORE, bn: Optional[int] = None,
          split: Optional[int] = None, deep: Optional[bool] = None, pdl: bool = False,
-         part_val=None, part_idx=None, part_lse=None, trace: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """``out = x @ w.T`` (+ ``residual``) on the tcgen05 kernel.  ``x (M, K)``, ``w (N, K)`` bf16."""
+         part_val=None, part_idx=None, part_lse=None, trace: Optional[torch.Tensor] = None,
+         pair: Optional[int] = None) -> torch.Tensor:
+    """``out = x @ w.T`` (+ ``residual``) on the tcgen05 kernel.  ``x (M, K)``, ``w (N, K)`` bf16.  ``pair``: width of
+    the tiles on CTA pairs (many rows; 0: single CTAs), from :func:`pick_pair_tile` when nothing else is asked for; ``bn``
+    is then the interleave of a SwiGLU weight."""
     lib = load()
     M, K = x.shape
     N = w.shape[0]
     assert w.shape[1] == K and x.stride(1) == 1 and w.stride(1) == 1
-    cb, cs, cd = pick_gemm_config(M, N, K, epi, bn)
-    bn = bn or cb
-    split = split or cs
-    deep = cd if deep is None else deep
+    if pair is None:
+        free = split is None and deep is None and trace is None and (bn is None or epi == EPI_SWIGLU)
+        pair = pick_pair_tile(M, N, K, bn or 128) if free and epi in (EPI_STORE, EPI_SWIGLU) and N % 8 == 0 else 0
+    if not pair:
+        cb, cs, cd = pick_gemm_config(M, N, K, epi, bn)
+        bn = bn or cb
+        split = split or cs
+        deep = cd if deep is None else deep
     if out is None:
         if epi == EPI_SWIGLU:
             out = torch.empty(M, N // 2, dtype=torch.bfloat16, device=x.device)
@@ -305,6 +334,11 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None,
         elif epi in (EPI_STORE,):
             out = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
     ldc = out.stride(0) if out is not None else 0
+    if pair:
+        _check(lib.js_gemm_pair(_p(x), _p(w), _p(out), _p(residual), M, N, K, x.stride(0), w.stride(0), ldc, epi, pair, (bn or 128) // 2,
+                                _p(part_val), _p(part_idx), _p(status_word(x.device)), int(pdl), _stream()),
+               f"js_gemm_pair(M={M},N={N},K={K},epi={epi})")
+        return out
     rc = lib.js_gemm_bf16(_p(x), _p(w), _p(out), _p(residual), M, N, K, x.stride(0), w.stride(0), ldc, epi, bn,
                           split, int(deep), _p(part_val), _p(part_idx), _p(part_lse),
                           _p(status_word(x.device)), _p(trace), int(pdl), _stream())
@@ -408,7 +442,8 @@ def lm_head_argmax(h: torch.Tensor, w: torch.Tensor, ws: Optional[dict] = None, 
     if ws is None:
         ws = {"val": torch.empty(M, nt, dtype=torch.float32, device=h.device),
               "idx": torch.empty(M, nt, dtype=torch.int32, device=h.device)}
-    gemm(h, w, out=None, epi=EPI_ARGMAX, bn=128, split=1, pdl=pdl, part_val=ws["val"], part_idx=ws["idx"])
+    gemm(h, w, out=None, epi=EPI_ARGMAX, bn=128, split=1, pdl=pdl, part_val=ws["val"], part_idx=ws["idx"],
+         pair=pick_pair_tile(M, N, h.shape[1]))
     if out_idx is None:
         out_idx = torch.empty(M, dtype=torch.int32, device=h.device)
     if out_val is None:
@@ -870,11 +905,14 @@ def gemm_inproj(x, w, raw: Optional[torch.Tensor], n_raw: int, act_out: Optional
     M, K = x.shape
     N = w.shape[0]
     if bn is None:
-        tiles2 = ((M + 127) // 128) * (N // 256)
-        if M >= 512 and N % 256 == 0 and tiles2 >= 64:
-            bn, split, deep = 256, 1, 0
-        else:
-            bn, split, deep = pick_gemm_config(M, N, K, EPI_SWIGLU, 128)
+        tn = pick_pair_tile(M, N, K)
+        if tn:
+            _check(lib.js_gemm_inproj_pair(_p(x), _p(w), _p(raw), _p(act_out), M, N, K, x.stride(0), w.stride(0),
+                                           raw.stride(0) if raw is not None else 0, act_out.stride(0) if act_out is not None else 0,
+                                           int(n_raw), int(act), *map(ctypes.c_float, act_args), tn, _p(status_word(x.device)), int(pdl),
+                                           _stream()), f"js_gemm_inproj_pair(M={M},N={N},K={K})")
+            return
+        bn, split, deep = pick_gemm_config(M, N, K, EPI_SWIGLU, 128)
     _check(lib.js_gemm_inproj(_p(x), _p(w), _p(raw), _p(act_out), M, N, K, x.stride(0), w.stride(0),
                               raw.stride(0) if raw is not None else 0, act_out.stride(0) if act_out is not None else 0,
                               int(n_raw), int(act), *map(ctypes.c_float, act_args), bn, split, int(deep), _p(status_word(x.device)), int(pdl),
@@ -888,11 +926,16 @@ def gemm_resid32(a, w, x: torch.Tensor, norm=None, h: Optional[torch.Tensor] = N
     lib = load()
     M, K = a.shape
     N = w.shape[0]
-    if bn is None:
-        bn, split, deep = pick_gemm_config(M, N, K, EPI_STORE)
-        if bn == 256 and deep != 3:
-            deep = 1
     nw, nb, alpha = norm if norm is not None else (None, None, 0.0)
+    if bn is None:
+        tn = pick_pair_tile(M, N, K)
+        if tn:
+            _check(lib.js_gemm_resid32_pair(_p(a), _p(w), _p(x), _p(x), M, N, K, a.stride(0), w.stride(0), x.stride(0), _p(emb),
+                                            emb.stride(0) if emb is not None else 0, _p(h), h.stride(0) if h is not None else 0,
+                                            _p(nw), _p(nb), ctypes.c_float(alpha), tn, _p(status_word(a.device)), int(pdl),
+                                            _stream()), f"js_gemm_resid32_pair(M={M},N={N},K={K})")
+            return
+        bn, split, deep = pick_gemm_config(M, N, K, EPI_STORE, 128)
     _check(lib.js_gemm_resid32(_p(a), _p(w), _p(x), _p(x), M, N, K, a.stride(0), w.stride(0), x.stride(0), _p(emb),
                                emb.stride(0) if emb is not None else 0, _p(h), h.stride(0) if h is not None else 0, _p(nw),
                                _p(nb), ctypes.c_float(alpha), bn, split, int(deep), _p(status_word(a.device)), int(pdl),

@@ -109,6 +109,60 @@ def test_gemm_last_row_tile(ext, M):
     ext.check_status("cuda")
 
 
+@pytest.mark.parametrize("M,N,K", [(129, 256, 64), (256, 384, 1000), (257, 640, 320), (300, 5000, 136), (1100, 4736, 256)])
+def test_gemm_on_cta_pairs(ext, M, N, K):
+    """Both tile widths of the CTA-pair GEMM at the edges of its 256-row tiles, K that ends inside a k-block or leaves the stages
+    half used, columns that end inside a tile, more tiles than pairs (two accumulators in turn), every epilogue, NaN behind
+    the last row."""
+    pad, w = rnd(M + 2, K, seed=50), rnd(N, K, scale=0.05, seed=51)
+    pad[M:] = float("nan")
+    x, r = pad[:M], rnd(M, N, seed=52)
+    ref = x.float() @ w.float().t()
+    for tile in (128, 256):
+        assert rel_err(ext.gemm(x, w, pair=tile), ref) < BF16_TOL
+        out = r.clone()
+        assert rel_err(ext.gemm(x, w, out=out, residual=out, pair=tile), ref + r.float()) < BF16_TOL
+        for bn in (128, 256):
+            if N % bn == 0 and bn <= tile:
+                act = ext.gemm(x, ext.interleave_gate_up(w[:N // 2], w[N // 2:], bn), epi=ext.EPI_SWIGLU, bn=bn, pair=tile)
+                assert rel_err(act, torch.nn.functional.silu(ref[:, :N // 2]) * ref[:, N // 2:]) < BF16_TOL
+        parts = (N + 127) // 128
+        val, idx = torch.empty(M, parts, device="cuda"), torch.empty(M, parts, dtype=torch.int32, device="cuda")
+        ext.gemm(x, w, epi=ext.EPI_ARGMAX, part_val=val, part_idx=idx, pair=tile)
+        full = torch.nn.functional.pad(ref, (0, parts * 128 - N), value=float("-inf")).view(M, parts, 128)
+        assert rel_err(val, full.amax(-1)) < 1e-4
+        assert rel_err(ref.gather(1, idx.long()), full.amax(-1)) < 1e-4
+    ext.check_status("cuda")
+
+
+@pytest.mark.parametrize("M", [200, 640])
+def test_inproj_and_resid32_on_cta_pairs(ext, M, monkeypatch):
+    K, N, n_raw = 192, 768, 256
+    x, w, wr = rnd(M, K, seed=60), rnd(N, K, scale=0.08, seed=61), rnd(N, K, scale=0.05, seed=62)
+    base, emb = torch.randn(M, N, device="cuda"), rnd(M, N, seed=63)
+    nw, nb = torch.randn(N, device="cuda"), torch.randn(N, device="cuda")
+    for tile in (128, 256, 0):
+        monkeypatch.setattr(ext, "pick_pair_tile", lambda *a, t=tile: t)
+        for act in (ext.ACT_GELU_GLU, ext.ACT_RELU2, ext.ACT_NONE, ext.ACT_GELU_ERF, ext.ACT_XIELU):
+            raw = torch.empty(M, n_raw, device="cuda")
+            out = torch.empty(M, (N - n_raw) // (2 if act == ext.ACT_GELU_GLU else 1), dtype=torch.bfloat16, device="cuda")
+            ext.gemm_inproj(x, w, raw, n_raw, out, False, act=act, act_args=(0.8, 0.3))
+            ref = x.float() @ w.float().t()
+            z = ref[:, n_raw:]
+            if act == ext.ACT_GELU_GLU:
+                b = z.view(M, -1, 2, 64)
+                want = (torch.nn.functional.gelu(b[:, :, 0], approximate="tanh") * b[:, :, 1]).reshape(M, -1)
+            else:
+                want = {ext.ACT_RELU2: lambda: z.relu() ** 2, ext.ACT_NONE: lambda: z, ext.ACT_GELU_ERF: lambda: torch.nn.functional.gelu(z),
+                        ext.ACT_XIELU: lambda: 0.5 * z + torch.where(z > 0, 0.8 * z * z, 0.3 * (z.exp() - 1 - z))}[act]()
+            assert rel_err(raw, ref[:, :n_raw]) < 1e-4 and rel_err(out, want) < BF16_TOL
+        y, h = base.clone(), torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+        ext.gemm_resid32(x, wr, y, norm=(nw, nb, 0.5), h=h, emb=emb)
+        want = base + x.float() @ wr.float().t() + emb.float()
+        assert rel_err(y, want) < 1e-4 and rel_err(h, torch.tanh(0.5 * want) * nw + nb) < BF16_TOL
+    ext.check_status("cuda")
+
+
 def test_gemm_fp32_out(ext):
     x, w = rnd(64, 512, seed=6), rnd(128, 512, scale=0.05, seed=7)
     out = ext.gemm(x, w, epi=ext.EPI_STORE_F32, split=2)
