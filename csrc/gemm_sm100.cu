@@ -70,7 +70,7 @@ struct GemmSmem {
   static constexpr int kBudget = BUDGET_KB * 1024;
   static constexpr int kMaxStages = FP4 ? 4 : 8;   // FP4: every stage also owns 32 tensor-memory columns of scales
   static constexpr int kStages = (kBudget / kStage) > kMaxStages ? kMaxStages : ((kBudget / kStage) < 2 ? 2 : (kBudget / kStage));
-  static constexpr int kMinBlocks = BUDGET_KB <= 100 ? 2 : 1;
+  static constexpr int kMinBlocks = BUDGET_KB <= 108 ? 2 : 1;
   static constexpr int kTiles = kStages * kStage;
 };
 
@@ -1028,10 +1028,15 @@ extern "C" int js_gemm_nvfp4(const void* Aq, const void* sfa, const float* row_s
   ActMaps ta;
   CUtensorMap tw;
   if (make_act_maps(&ta, &p, Aq, K / 2, lda_bytes, true) || make_map_u8(&tw, Wq, N, K / 2, ldw_bytes, 128)) return -16;
+  // More tiles than SMs: three stages (108 KB, 256 tensor-memory columns), so that two CTAs share an SM and one's
+  // epilogue runs under the other's loads.  192 tiles of a 24576 x 4096 gate/up ran as two rounds of one CTA per SM: 30.1 us
+  // at 64 rows, 16.4 this way; 325 and 155 at 2048 rows.
+  const bool shared_sm = split == 1 && ((N + 127) / 128) * ((M + BM - 1) / BM) > 148;
 #define JS_CASE4(EPI_)                                                                                   \
   if (epi == EPI_)                                                                                        \
-    return split > 1 ? launch_gemm<128, EPI_, 128, true>(ta, tw, p, split, pdl != 0, stream)              \
-                     : launch_gemm<128, EPI_, 160, true>(ta, tw, p, split, pdl != 0, stream);
+    return split > 1   ? launch_gemm<128, EPI_, 128, true>(ta, tw, p, split, pdl != 0, stream)            \
+           : shared_sm ? launch_gemm<128, EPI_, 108, true>(ta, tw, p, 1, pdl != 0, stream)                \
+                       : launch_gemm<128, EPI_, 160, true>(ta, tw, p, 1, pdl != 0, stream);
   JS_CASE4(EPI_STORE) JS_CASE4(EPI_SWIGLU) JS_CASE4(EPI_STORE_F32)
 #undef JS_CASE4
   return -17;
