@@ -1090,8 +1090,11 @@ class FastRound:
         ids32 = torch.cat([p.reshape(-1) for p in prompts]).to(device=dev, dtype=torch.int32)
         rows = [pool.state(sid).row for sid in sids]
         last = cfg.num_hidden_layers - 1
-        for s0 in range(0, total, _PREFILL_ROWS):
-            n = min(_PREFILL_ROWS, total - s0)
+        portion = _PREFILL_ROWS
+        if cfg.is_moe:                      # what the routing kernels sort in one launch
+            portion = max(1, min(portion, 16384 // cfg.num_experts_per_tok))
+        for s0 in range(0, total, portion):
+            n = min(portion, total - s0)
             parts = []                                  # (prompt, its first token here, tokens)
             for i, (end, length) in enumerate(zip(ends, lens)):
                 lo, hi = max(s0, end - length), min(s0 + n, end)
@@ -1104,7 +1107,7 @@ class FastRound:
                                                                            dtype=np.int32)))).to(dev)
             pos, seq, cu_q, seq_rows, past = meta.split([n, n, len(parts) + 1, len(parts), len(parts)])
             slots = pool.slot_map[seq.long(), pos.long()]
-            st = _Stack(self.lcfg, n, dev, pool.max_seq_len)
+            st = _Stack(self.lcfg, n, dev, pool.max_seq_len, len(parts))
             tapbuf = hidden[s0:s0 + n] if hidden is not None else None
             X.embed(ids32[s0:s0 + n], self.embed_w, out=st.x)
             xn = torch.empty_like(st.x)
