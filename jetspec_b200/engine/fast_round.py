@@ -114,20 +114,10 @@ def _finish_layer_weights(out: list) -> list:
 _PREFILL_ROWS = 2048
 
 
-def _gu_wide(L: dict) -> torch.Tensor:
-    """The layer's gate/up weight re-interleaved for 256-column tiles (128 gate + 128 up rows per tile)."""
-    if "gu256" not in L:
-        w, h = L["gu"], L.get("gu_bn", 128) // 2
-        I2, H = w.shape
-        v = w.view(I2 // (2 * h), 2, h, H)
-        L["gu256"] = X.interleave_gate_up(v[:, 0].reshape(I2 // 2, H), v[:, 1].reshape(I2 // 2, H), 256)
-    return L["gu256"]
-
-
 class _Stack:
-    """Static activation buffers of one decoder stack for a fixed row count ``T``."""
+    """Static activation buffers of one decoder stack for a fixed row count ``T`` of ``seqs`` sequences."""
 
-    def __init__(self, cfg, T: int, device, max_keys: int):
+    def __init__(self, cfg, T: int, device, max_keys: int, seqs: int = 1):
         H, I = cfg.hidden_size, cfg.intermediate_size
         Hq, Hkv, D = cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim
         bf = dict(dtype=torch.bfloat16, device=device)
@@ -139,7 +129,7 @@ class _Stack:
         self.attn = torch.zeros(T, Hq * D, **bf)
         self.act = torch.zeros(T, I, **bf)
         self._q4: dict = {}
-        self.splits = X.attn_splits_for(T, Hq, Hkv, max_keys)
+        self.splits = X.attn_splits_for(T, Hq, Hkv, max_keys, seqs)
         self.attn_ws = None
         if self.splits > 1:
             self.attn_ws = {"o": torch.zeros(self.splits, T, Hq, D, dtype=torch.float32, device=device),
@@ -375,10 +365,10 @@ class FastRound:
         self._tp_graph_key = None
 
     # ------------------------------------------------------------------ decoder stack (either model family)
-    def _new_stack(self, T: int, max_keys: int):
+    def _new_stack(self, T: int, max_keys: int, seqs: int = 1):
         if self.stack is not None:
             return self.stack.buffers(T, max_keys)
-        return _Stack(self.lcfg, T, self.device, max_keys)
+        return _Stack(self.lcfg, T, self.device, max_keys, seqs)
 
     def _run_stack(self, st, ids, seq_rows, cu_q, past, positions, slots, mask, causal: bool, max_q: int, xn, taps=None,
                    tap_ids=None, pdl: bool = True, embed_pdl: bool = True, prefetch=None, state_rows=None) -> int:
@@ -831,7 +821,7 @@ class FastRound:
             r["ar"] = torch.arange(NB, dtype=torch.long, device=dev)
             r["greedy"] = _i32(T, dev)
             r["greedy_host"] = torch.zeros(T, dtype=torch.int32).pin_memory()
-            r["stack"] = self._new_stack(T, pool.max_seq_len)
+            r["stack"] = self._new_stack(T, pool.max_seq_len, T // NB)
             r["xn"] = torch.zeros(T, self.xn_cols, dtype=torch.bfloat16, device=dev)
             nt = X.n_tiles(self.lm_head_w.shape[0])
             r["am_ws"] = {"val": torch.zeros(T, nt, dtype=torch.float32, device=dev),
