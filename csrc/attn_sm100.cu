@@ -310,8 +310,8 @@ __global__ void attn_merge_kernel(AttnParams p) {
   float acc[4] = {0.f, 0.f, 0.f, 0.f}, l = 0.f;
   for (int s = 0; s < p.splits; ++s) {
     const float ms = p.ws_ml[(s * stride + row) * 2], ls = p.ws_ml[(s * stride + row) * 2 + 1];
-    if (ms == -INFINITY) continue;   // this split saw no visible key (its O may be unwritten)
-    const float w = exp2f(ms - m);
+    if (ls == 0.f) continue;         // this split saw no visible key (its O may be unwritten)
+    const float w = exp2f(ms - (m == -INFINITY ? 0.f : m));   // NaN scores leave a sum without a maximum
     l += ls * w;
     const float4 v = *reinterpret_cast<const float4*>(p.ws_o + (s * stride + row) * AD + lane * 4);
     acc[0] += v.x * w; acc[1] += v.y * w; acc[2] += v.z * w; acc[3] += v.w * w;

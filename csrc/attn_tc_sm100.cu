@@ -11,8 +11,10 @@
 //     live in tensor memory, so the softmax threads own one ROW each (no shuffles): they read S with
 //     tcgen05.ld, write P as bf16 into a swizzled shared-memory tile that feeds the second MMA, and
 //     rescale O in tensor memory only when a row's integer running maximum grows;
-//   * K/V rows are gathered by slot with cp.async into 128-byte-swizzled tiles (three stages) by four
-//     loader warps; V is consumed as an MN-major operand, so no transpose is ever made;
+//   * K/V rows are fetched by slot into 128-byte-swizzled tiles (a ring of stages); V is consumed as an MN-major operand, so
+//     no transpose is ever made.  kPlain and kTwo fetch by TMA: four loader warps take 16 keys of a tile each, one box of 16
+//     rows where their slots follow one another (a page), gathers of four rows where they do not.  The other forms gather
+//     with cp.async, which took 0.5 to 1 us of a loader's time per 64-key tile and held a CTA to about 30 GB/s;
 //   * warp 4 issues all MMAs: QK(t+1) is issued before PV(t), so the tensor pipe works on the next
 //     scores while the softmax of the current tile runs.
 //
@@ -23,10 +25,16 @@
 //   * kPlain: the above, with an optional window, kept first tokens, sinks and gates;
 //   * kPooled: scores may be capped, and tiles of pooled blocks (one key and value per P tokens, read through a block map)
 //     stand ahead of the window's tiles;
+//   * kTwo: kPlain with two softmax groups (warps 0-3 and 4-7) that take every other key tile, each with its own running
+//     maximum, sum and output accumulator; the two halves meet in the epilogue.  One group's chain per tile (scores out of
+//     tensor memory, maximum, exponentials, probabilities into shared memory) takes about 1.2 us while a tile's MMAs
+//     take 0.25 us, so a launch with many tiles per CTA was bound by that chain, and next by the cp.async loaders.
+//     128-node trees of 32 query and 8 KV heads, before / after (us): 4 sequences of 2048 - 12000 keys 241 / 150, 16 of
+//     3000 - 12000 636 / 393, 16 of 300 - 2048 156 / 107; 3 x 600 causal rows behind up to 5000 keys 335 / 204;
 //   * kDiff: two attention maps a head over the same values.  Query and key rows hold 64 columns for each map, so a tile's K
 //     and V are gathered once and give two score tiles and two outputs (warps 0-3 and 4-7 own one map each, warp 8
 //     issues, four loader warps); the epilogue (or the merge of the key splits) norms o1 - lam o2.
-#include "common.cuh"
+#include "gemm_common.cuh"
 
 #include <math.h>
 #include <type_traits>
@@ -36,22 +44,39 @@ namespace js {
 constexpr int TD = 128;          // head dim
 constexpr int TROWS = 128;       // query rows per CTA
 constexpr int TKEYS = 64;        // keys per tile
-constexpr int TSTAGES = 3;
 constexpr int TTHREADS = 416;       // softmax threads of every map, one issuing warp, loaders
-enum AttnMode : int { kPlain = 0, kPooled = 1, kDiff = 2 };
+enum AttnMode : int { kPlain = 0, kPooled = 1, kDiff = 2, kTwo = 3 };
 // loader threads (gather throughput grows with the copies in flight)
-__host__ __device__ constexpr int loader_threads(int mode) { return TTHREADS - 32 - (mode == kDiff ? 256 : 128); }
+__host__ __device__ constexpr int softmax_groups(int mode) { return mode == kDiff || mode == kTwo ? 2 : 1; }
+__host__ __device__ constexpr int loader_threads(int mode) { return TTHREADS - 32 - 128 * softmax_groups(mode); }
 __host__ __device__ constexpr int attn_maps(int mode) { return mode == kDiff ? 2 : 1; }
+__host__ __device__ constexpr bool attn_tma(int mode) { return mode == kPlain || mode == kTwo; }
+__host__ __device__ constexpr int attn_stages(int mode) { return attn_tma(mode) ? 5 : 3; }      // as many as fit where TMA fills them
 constexpr int kStageKV = 2 * TKEYS * 256;      // K then V, each 2 halves x 64 keys x 128 B
 constexpr int kSmemQ = TROWS * 256;            // 2 halves x 128 rows x 128 B
 constexpr int kSmemP = TROWS * 128;            // 128 rows x 64 keys bf16
-constexpr int attn_tc_smem(int mode) { return kSmemQ + TSTAGES * kStageKV + 2 * attn_maps(mode) * kSmemP + 256 + 1024; }
+constexpr int attn_tc_smem(int mode) { return kSmemQ + attn_stages(mode) * kStageKV + 2 * attn_maps(mode) * kSmemP + 256 + 1024; }
 // Key splits that merge inside a cluster (portable cluster size); the chunk receive area must fit the dead
 // K/V stages + P buffers, the (max, sum) pairs the dead Q tile.
 constexpr int kMaxClusterSplits = 8;
-static_assert(kMaxClusterSplits * 16384 <= TSTAGES * kStageKV + 2 * kSmemP, "chunk receive area");
-static_assert(3 * 2 * 16384 <= TSTAGES * kStageKV + 2 * kSmemP, "chunk receive area, 3 splits own 2 chunks each");
+static_assert(kMaxClusterSplits * 16384 <= attn_stages(kPlain) * kStageKV + 2 * kSmemP, "chunk receive area");
+static_assert(3 * 2 * 16384 <= attn_stages(kPlain) * kStageKV + 2 * kSmemP, "chunk receive area, 3 splits own 2 chunks each");
 static_assert(kMaxClusterSplits * TROWS * 8 <= kSmemQ, "(max, sum) receive area");
+
+// kPlain, kTwo: tensor maps of the pools.  Head h's slot s is row h * head_rows + s, from column h * head_cols.
+struct AttnMaps {
+  CUtensorMap k16, v16;        // boxes of 16 rows x 64 columns
+  CUtensorMap k1, v1;          // boxes of one row, for gathers
+  int head_rows, head_cols;
+};
+
+// Four rows of 64 columns each into 512 consecutive bytes (x a multiple of 8, the map's box one row high).
+JS_DEVICE void tma_gather4(uint32_t dst, const CUtensorMap* m, uint64_t* bar, int x, int y0, int y1, int y2, int y3) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(x), "r"(y0), "r"(y1), "r"(y2), "r"(y3)
+      : "memory");
+}
 
 struct AttnTcParams {
   const __nv_bfloat16* q;      // (T, Hq, 128)
@@ -126,10 +151,46 @@ JS_DEVICE bool mbar_wait_backoff(uint64_t* bar, uint32_t parity, int* status, in
   report(status, code);
   return false;
 }
+// The waits of the kernel's roles: without cp.async loaders nothing is disturbed by a suspended try_wait.
+template <bool TMA>
+JS_DEVICE bool attn_wait(uint64_t* bar, uint32_t parity, int* status, int code) {
+  return TMA ? mbar_wait(bar, parity, status, code) : mbar_wait_backoff(bar, parity, status, code);
+}
+JS_DEVICE void tma_load_2d_at(uint32_t dst, const CUtensorMap* m, uint64_t* bar, int x, int y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(x), "r"(y)
+      : "memory");
+}
 JS_DEVICE float fast_exp2(float x) {     // 2^x, flushing denormal results to zero; exp2(-inf) = 0
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+// AND over the `n` threads of named barrier 1
+JS_DEVICE bool named_and(bool pred, int n) {
+  int out;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 q, %1, 0;\n\tbar.red.and.pred p, 1, %2, q;\n\tselp.s32 %0, 1, 0, p;\n\t}"
+      : "=r"(out) : "r"(static_cast<int>(pred)), "r"(n) : "memory");
+  return out != 0;
+}
+// two fp32 in one register pair: half as many instructions per score
+JS_DEVICE uint64_t pack_f32x2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+JS_DEVICE void unpack_f32x2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+JS_DEVICE uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+JS_DEVICE uint64_t add_f32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
 }
 JS_DEVICE void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
@@ -159,9 +220,13 @@ JS_DEVICE void attn_trace(int slot) {
 }
 
 template <int G, int MODE>
-__global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcParams p) {
+__global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcParams p, const __grid_constant__ AttnMaps maps) {
+  constexpr bool TMA = attn_tma(MODE);
   constexpr int NPT = TROWS / G;   // nodes per q tile
-  constexpr int MAPS = attn_maps(MODE), TLOADERS = loader_threads(MODE), MMA_WARP = 4 * MAPS;
+  constexpr int MAPS = attn_maps(MODE), GROUPS = softmax_groups(MODE), TLOADERS = loader_threads(MODE), MMA_WARP = 4 * GROUPS;
+  constexpr int TSTAGES = attn_stages(MODE);
+  // Tile i of a map uses score buffer (and barriers) i % NB and probability buffer i % 2; PV follows QK by LAG tiles.
+  constexpr int LAG = MODE == kTwo ? 2 : 1, NB = 2 * LAG, NBSH = MODE == kTwo ? 2 : 1;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
@@ -171,10 +236,10 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
   uint64_t* q_full = bars;                 // 1
   uint64_t* kv_full = bars + 1;            // TSTAGES
   uint64_t* kv_empty = kv_full + TSTAGES;  // TSTAGES
-  uint64_t* s_full = kv_empty + TSTAGES;   // 2 a map
-  uint64_t* p_full = s_full + 2 * MAPS;    // 2 a map
-  uint64_t* pv_done = p_full + 2 * MAPS;   // 2 a map
-  uint64_t* o_done = pv_done + 2 * MAPS;   // 1
+  uint64_t* s_full = kv_empty + TSTAGES;   // NB a map
+  uint64_t* p_full = s_full + NB * MAPS;   // NB a map
+  uint64_t* pv_done = p_full + NB * MAPS;  // NB a map
+  uint64_t* o_done = pv_done + NB * MAPS;  // 1
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -234,11 +299,12 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
   const size_t out_row = static_cast<size_t>(q_begin + (row_valid ? node : 0)) * p.Hq + head;
   __nv_bfloat16* out_ptr = p.out + static_cast<size_t>(q_begin + (row_valid ? node : 0)) * p.ldo + head * TD;
 
-  const bool cmerge = MODE != kDiff && p.cluster_merge != 0;
+  const bool cmerge = GROUPS == 1 && p.cluster_merge != 0;
   const int map = MODE == kDiff ? warp >> 2 : 0;      // softmax threads: the map they own
-  const bool softmax_warp = warp < 4 * MAPS;
+  const int group = MODE == kTwo ? warp >> 2 : 0;     // kTwo: tiles group, group + 2, ...
+  const bool softmax_warp = warp < 4 * GROUPS;
   float m_run = -INFINITY, l_run = 0.f;     // softmax threads: running (integer) maximum and sum of their row
-  if (p.sink && split == p.splits - 1) {    // the last split always has a tile
+  if (p.sink && split == p.splits - 1 && group == 0) {    // the last split always has a tile
     const float s2 = p.sinks != nullptr && row_valid ? p.sinks[head] * 1.4426950408889634f : 0.f;
     m_run = ceilf(s2);
     l_run = exp2f(s2 - m_run);
@@ -256,13 +322,13 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
 
   if (tid == 0 && nt > 0) {
     mbar_init(q_full, TLOADERS);
-    for (int s = 0; s < TSTAGES; ++s) { mbar_init(&kv_full[s], TLOADERS); mbar_init(&kv_empty[s], 1); }
-    for (int i = 0; i < 2 * MAPS; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 128); mbar_init(&pv_done[i], 1); }
+    for (int s = 0; s < TSTAGES; ++s) { mbar_init(&kv_full[s], TMA ? 4 : TLOADERS); mbar_init(&kv_empty[s], 1); }
+    for (int i = 0; i < NB * MAPS; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 128); mbar_init(&pv_done[i], 1); }
     mbar_init(o_done, 1);
     fence_barrier_init();
   }
   if (warp == MMA_WARP && nt > 0) {
-    tmem_alloc(tmem_slot, 256 * MAPS);
+    tmem_alloc(tmem_slot, 256 * GROUPS);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -270,7 +336,7 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
   tc_fence_after();
   const uint32_t tmem_base = nt > 0 ? *tmem_slot : 0u;
   if (tid == 0) attn_trace(1);      // setup done
-  const uint32_t tmem_o = tmem_base + 128 * MAPS;      // map m: S buffers at columns 128 m and 128 m + 64, O behind all of them
+  const uint32_t tmem_o = tmem_base + 128 * GROUPS;    // S buffers of map m at columns 128 m + 64 b, O of every map or group behind them all
 
   const uint32_t t_lane = static_cast<uint32_t>((warp & 3) * 32) << 16;
   if (nt <= 0) {
@@ -287,6 +353,65 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
       cp_async16_tc(q_addr + (ch >> 3) * (TROWS * 128) + r * 128 + (((ch & 7) ^ (r & 7)) << 4), src, valid);
     }
     cp_async_commit_tc();
+    if constexpr (TMA) {
+      auto q_landed = [&] {
+        cp_async_wait_tc<0>();
+        fence_proxy_async();
+        mbar_arrive(q_full);
+      };
+      const int lw = lt >> 5;                   // loader warps 0..3: keys 16 lw .. of every tile
+      if (lw < 4) {
+        // slot of this lane's key; keys past the end repeat the last one (no row sees them)
+        auto slot_at = [&](int i) { return __ldg(slots + min(tile_key(i) + 16 * lw + (lane & 15), L - 1)); };
+        const int row0 = h * maps.head_rows, x0 = h * maps.head_cols;
+        int next = slot_at(0), s = 0;
+        uint32_t phase = 1;                     // of kv_empty: the first round finds every stage free
+        bool ok = true;
+        for (int i = 0; i < nt; ++i) {
+          int slot = next;
+          if (i + 1 < nt) next = slot_at(i + 1);
+          if (slot < 0 || slot >= p.S) { report(p.status, kBadSlot); slot = 0; }
+          ok = attn_wait<TMA>(&kv_empty[s], phase, p.status, kTimeoutEmpty);
+          if (!ok) break;
+          const uint32_t dst = smem_u32(sKV + s * kStageKV) + lw * (16 * 128);
+          const int first = __shfl_sync(0xffffffffu, slot, 0);
+          const bool page = __all_sync(0xffffffffu, slot == first + (lane & 15));
+          if (elect_one()) mbar_expect_tx(&kv_full[s], 16 * 512);
+          __syncwarp();
+          if (page) {
+            if (elect_one()) {
+#pragma unroll
+              for (int half = 0; half < 2; ++half) {
+                tma_load_2d_at(dst + half * (TKEYS * 128), &maps.k16, &kv_full[s], x0 + half * 64, row0 + first);
+                tma_load_2d_at(dst + TKEYS * 256 + half * (TKEYS * 128), &maps.v16, &kv_full[s], x0 + half * 64, row0 + first);
+              }
+            }
+          } else {
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+              int y[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) y[e] = row0 + __shfl_sync(0xffffffffu, slot, 4 * g + e);
+              if (elect_one()) {
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                  const uint32_t at = dst + g * 512 + half * (TKEYS * 128);
+                  tma_gather4(at, &maps.k1, &kv_full[s], x0 + half * 64, y[0], y[1], y[2], y[3]);
+                  tma_gather4(at + TKEYS * 256, &maps.v1, &kv_full[s], x0 + half * 64, y[0], y[1], y[2], y[3]);
+                }
+              }
+              __syncwarp();
+            }
+          }
+          __syncwarp();
+          if (lane == 0 && lw == 0 && i < 8) attn_trace(32 + i);    // copies of tile i issued
+          if (i == 0) q_landed();
+          if (++s == TSTAGES) { s = 0; phase ^= 1; }
+        }
+      } else {
+        q_landed();
+      }
+    } else {
     constexpr int RSTEP = TLOADERS / 16;        // key rows covered by one pass of all loader threads
     const int ch = lt & 15, r0 = lt >> 4;       // this thread copies chunk `ch` of keys r0, r0+RSTEP, ...
     // slots of the first tile; the next tile's are fetched while the current tile's copies are issued
@@ -320,7 +445,7 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
           // about to block on the consumer: it may itself be waiting for tiles not yet published
           cp_async_wait_tc<0>();
           publish_before(i);
-          ok = mbar_wait_backoff(&kv_empty[s], par, p.status, kTimeoutEmpty);
+          ok = attn_wait<TMA>(&kv_empty[s], par, p.status, kTimeoutEmpty);
         }
       }
       if (!ok) break;
@@ -365,54 +490,61 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
       cp_async_wait_tc<0>();
       publish_before(nt);
     }
+    }
   } else if (warp == MMA_WARP) {
     // ================================================================ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc_qk = umma_idesc_bf16(TROWS, TKEYS);
-      constexpr uint32_t idesc_pv = umma_idesc_bf16_bmn(TROWS, TD);
-      bool ok = mbar_wait_backoff(q_full, 0, p.status, kTimeoutFull);
-      attn_trace(2);                // Q landed
-      // O += P V of tile j for every map, each as soon as its P is there
-      auto issue_pv = [&](int j) {
-        const int s = j % TSTAGES, pb = j & 1;
-        const uint32_t v_addr = smem_u32(sKV + s * kStageKV + TKEYS * 256);
+    // All lanes run the loop and one elected lane issues (see gemm_bf16_kernel).
+    constexpr uint32_t idesc_qk = umma_idesc_bf16(TROWS, TKEYS);
+    constexpr uint32_t idesc_pv = umma_idesc_bf16_bmn(TROWS, TD);
+    const uint64_t q_desc = umma_desc_sw128(smem_u32(sQ)), k_desc = umma_desc_sw128(smem_u32(sKV)),
+                   p_desc = umma_desc_sw128(smem_u32(sP)), v_desc = umma_desc_sw128_mn(smem_u32(sKV) + TKEYS * 256, TKEYS * 128);
+    bool ok = attn_wait<TMA>(q_full, 0, p.status, kTimeoutFull);
+    if (lane == 0) attn_trace(2);                // Q landed
+    // O += P V of tile j for every map, each as soon as its P is there
+    auto issue_pv = [&](int j) {
+      const int s = j % TSTAGES, pb = j & (NB - 1);
+      const uint32_t acc = tmem_o + (MODE == kTwo ? (j & 1) * TD : 0);
 #pragma unroll
-        for (int m = 0; m < MAPS; ++m) {
-          if (!mbar_wait_backoff(&p_full[2 * m + pb], (j >> 1) & 1, p.status, kTimeoutAccum)) return false;
-          tc_fence_after();
-          const uint64_t a_desc = umma_desc_sw128(smem_u32(sP + (2 * m + pb) * kSmemP));
+      for (int m = 0; m < MAPS; ++m) {
+        if (!attn_wait<TMA>(&p_full[NB * m + pb], (j >> NBSH) & 1, p.status, kTimeoutAccum)) return false;
+        tc_fence_after();
+        if (elect_one()) {
+          const uint64_t a_desc = p_desc + static_cast<uint64_t>((2 * m + (j & 1)) * (kSmemP >> 4));
+          const uint64_t b_desc = v_desc + static_cast<uint64_t>(s * (kStageKV >> 4));
 #pragma unroll
           for (int k = 0; k < TKEYS / 16; ++k)
-            umma_f16(tmem_o + m * TD, a_desc + 2 * k, umma_desc_sw128_mn(v_addr + k * 2048, TKEYS * 128), idesc_pv, (j | k) != 0 ? 1u : 0u);
+            umma_f16(acc + m * TD, a_desc + 2 * k, b_desc + k * (2048 >> 4), idesc_pv, k > 0 || j >= LAG ? 1u : 0u);
           if (m == MAPS - 1) umma_commit(&kv_empty[s]);
-          umma_commit(&pv_done[2 * m + pb]);
+          umma_commit(&pv_done[NB * m + pb]);
         }
-        return true;
-      };
-      for (int i = 0; i < nt && ok; ++i) {
-        const int s = i % TSTAGES, sb = i & 1;
-        ok = mbar_wait_backoff(&kv_full[s], (i / TSTAGES) & 1, p.status, kTimeoutFull);
-        if (!ok) break;
-        if (i < 8) attn_trace(8 + i);   // K/V tile i landed
-        // S buffer sb was consumed when P of tile i-2 was published (waited for below, before PV(i-2))
-        tc_fence_after();
-        const uint32_t k_addr = smem_u32(sKV + s * kStageKV);
+        __syncwarp();
+      }
+      return true;
+    };
+    for (int i = 0; i < nt && ok; ++i) {
+      const int s = i % TSTAGES, sb = i & (NB - 1);
+      ok = attn_wait<TMA>(&kv_full[s], (i / TSTAGES) & 1, p.status, kTimeoutFull);
+      if (!ok) break;
+      if (lane == 0 && i < 8) attn_trace(8 + i);   // K/V tile i landed
+      // S buffer sb was consumed when P of tile i - NB was published (waited for before PV(i - NB), issued at step i - LAG)
+      tc_fence_after();
+      if (elect_one()) {
+        const uint64_t b_desc = k_desc + static_cast<uint64_t>(s * (kStageKV >> 4));
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const uint32_t hoff = (k >> 2), kk = k & 3;          // each half of the columns is a map of its own in kDiff
-          umma_f16(tmem_base + (MAPS == 2 ? hoff * 2 * TKEYS : 0) + sb * TKEYS, umma_desc_sw128(smem_u32(sQ) + hoff * (TROWS * 128)) + 2 * kk,
-                   umma_desc_sw128(k_addr + hoff * (TKEYS * 128)) + 2 * kk, idesc_qk, (MAPS == 2 ? kk : k) != 0 ? 1u : 0u);
+          umma_f16(tmem_base + (MAPS == 2 ? hoff * 2 * TKEYS : 0) + sb * TKEYS, q_desc + hoff * (TROWS * 128 >> 4) + 2 * kk,
+                   b_desc + hoff * (TKEYS * 128 >> 4) + 2 * kk, idesc_qk, (MAPS == 2 ? kk : k) != 0 ? 1u : 0u);
           if (MAPS == 2 && k == 3) umma_commit(&s_full[sb]);
         }
-        umma_commit(&s_full[2 * (MAPS - 1) + sb]);
-        if (i >= 1) {
-          ok = issue_pv(i - 1);
-          if (!ok) break;
-        }
+        umma_commit(&s_full[NB * (MAPS - 1) + sb]);
       }
-      if (ok) ok = issue_pv(nt - 1);
-      umma_commit(o_done);     // also releases the epilogue on an error path
+      __syncwarp();
+      if (i >= LAG) ok = issue_pv(i - LAG);
     }
+    for (int j = max(0, nt - LAG); j < nt && ok; ++j) ok = issue_pv(j);
+    if (elect_one()) umma_commit(o_done);     // also releases the epilogue on an error path
+    __syncwarp();
   } else {
     // ================================================================ softmax + epilogue (one row per thread)
     int mw[8];
@@ -445,15 +577,15 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
       }
     }
     bool ok = true;
-    for (int i = 0; i < nt && ok; ++i) {
-      const int sb = i & 1;
-      ok = mbar_wait_backoff(&s_full[2 * map + sb], (i >> 1) & 1, p.status, kTimeoutAccum);
+    for (int i = group; i < nt && ok; i += LAG) {
+      const int sb = i & (NB - 1), buf = NB * map + sb;
+      ok = attn_wait<TMA>(&s_full[buf], (i >> NBSH) & 1, p.status, kTimeoutAccum);
       if (!ok) break;
       tc_fence_after();
       if (tid == 0 && i < 8) attn_trace(16 + i);   // scores of tile i ready
       uint32_t sr[64];
-      tmem_ld_32x32(tmem_base + t_lane + (2 * map + sb) * TKEYS, sr);
-      tmem_ld_32x32(tmem_base + t_lane + (2 * map + sb) * TKEYS + 32, sr + 32);
+      tmem_ld_32x32(tmem_base + t_lane + buf * TKEYS, sr);
+      tmem_ld_32x32(tmem_base + t_lane + buf * TKEYS + 32, sr + 32);
       tmem_ld_wait();
       // visibility of the tile's 64 keys for this row, as one 64-bit word (bit c = key k0 + c)
       const int k0 = tile_key(i);
@@ -498,73 +630,74 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
           to_log2 = 1.f;
         }
       }
-      if (vm == ~0ull) {              // the common case: every key of the tile is visible to this row
+      if (to_log2 <= 0.f) {           // the maximum below is taken before scaling
 #pragma unroll
-        for (int c = 0; c < 64; ++c) {
-          const float x = __uint_as_float(sr[c]) * to_log2;
-          sr[c] = __float_as_uint(x);
-          mx4[c & 3] = fmaxf(mx4[c & 3], x);
-        }
-      } else {
-#pragma unroll
-        for (int c = 0; c < 64; ++c) {
-          const bool vis = (vm >> c) & 1ull;
-          const float x = vis ? __uint_as_float(sr[c]) * to_log2 : -INFINITY;
-          sr[c] = __float_as_uint(x);
-          mx4[c & 3] = fmaxf(mx4[c & 3], x);
-        }
+        for (int c = 0; c < 64; ++c) sr[c] = __float_as_uint(__uint_as_float(sr[c]) * to_log2);
+        to_log2 = 1.f;
       }
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+      if (vm != ~0ull) {              // commonly every key of the tile is visible to this row
+#pragma unroll
+        for (int c = 0; c < 64; ++c)
+          if (!((vm >> c) & 1ull)) sr[c] = 0xff800000u;       // -inf
+      }
+#pragma unroll
+      for (int c = 0; c < 64; ++c) mx4[c & 3] = fmaxf(mx4[c & 3], __uint_as_float(sr[c]));
+      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * to_log2;
       // integer running maximum in the log2 domain (probabilities are then exact powers of two apart
       // whatever the tile order or key split; see the mma.sync kernel)
       const float m_new = fmaxf(m_run, ceilf(mx));
       const float m_safe = (m_new == -INFINITY) ? 0.f : m_new;
       const float alpha = exp2f(m_run - m_safe);          // 0 when nothing was visible before
       m_run = m_new;
-      // P buffer sb is free once PV of tile i-2 has completed
-      if (i >= 2) ok = mbar_wait_backoff(&pv_done[2 * map + sb], ((i - 2) >> 1) & 1, p.status, kTimeoutAccum);
+      // the P buffer is free once PV of tile i - 2 has completed
+      if (i >= 2) ok = attn_wait<TMA>(&pv_done[NB * map + ((i - 2) & (NB - 1))], ((i - 2) >> NBSH) & 1, p.status, kTimeoutAccum);
       if (!ok) break;
-      float rs4[4] = {0.f, 0.f, 0.f, 0.f};
-      const uint32_t p_row = smem_u32(sP + (2 * map + sb) * kSmemP) + row * 128;
+      const uint64_t scale2 = pack_f32x2(to_log2, to_log2), shift2 = pack_f32x2(-m_safe, -m_safe);
+      uint64_t rs2[4] = {0ull, 0ull, 0ull, 0ull};         // pairs of partial sums
+      const uint32_t p_row = smem_u32(sP + (2 * map + (i & 1)) * kSmemP) + row * 128;
 #pragma unroll
       for (int c8 = 0; c8 < 8; ++c8) {
         uint32_t w4[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float p0 = fast_exp2(__uint_as_float(sr[c8 * 8 + 2 * e]) - m_safe);
-          const float p1 = fast_exp2(__uint_as_float(sr[c8 * 8 + 2 * e + 1]) - m_safe);
-          rs4[e] += p0 + p1;
+          float p0, p1;
+          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sr[c8 * 8 + 2 * e]), __uint_as_float(sr[c8 * 8 + 2 * e + 1])), scale2, shift2), p0, p1);
+          p0 = fast_exp2(p0);
+          p1 = fast_exp2(p1);
+          rs2[e] = add_f32x2(rs2[e], pack_f32x2(p0, p1));
           __nv_bfloat162 v = __floats2bfloat162_rn(p0, p1);
           w4[e] = *reinterpret_cast<uint32_t*>(&v);
         }
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(p_row + ((c8 ^ (row & 7)) << 4)), "r"(w4[0]),
                      "r"(w4[1]), "r"(w4[2]), "r"(w4[3]) : "memory");
       }
-      l_run = l_run * alpha + ((rs4[0] + rs4[1]) + (rs4[2] + rs4[3]));
+      float rs_lo, rs_hi;
+      unpack_f32x2(add_f32x2(add_f32x2(rs2[0], rs2[1]), add_f32x2(rs2[2], rs2[3])), rs_lo, rs_hi);
+      l_run = l_run * alpha + (rs_lo + rs_hi);
       // rescale O when some row of this warp raised its maximum (tcgen05.ld/st are warp-wide)
-      const bool need = i > 0 && alpha != 1.f;
+      const bool need = i >= LAG && alpha != 1.f;
       if (__any_sync(0xffffffffu, need)) {
-        ok = mbar_wait_backoff(&pv_done[2 * map + ((i - 1) & 1)], ((i - 1) >> 1) & 1, p.status, kTimeoutAccum);   // every earlier PV is in O
+        ok = attn_wait<TMA>(&pv_done[NB * map + ((i - LAG) & (NB - 1))], ((i - LAG) >> NBSH) & 1, p.status, kTimeoutAccum);   // every earlier PV is in O
         if (!ok) break;
         tc_fence_after();
 #pragma unroll 1
         for (int c0 = 0; c0 < TD; c0 += 32) {
           uint32_t orr[32];
-          tmem_ld_32x32(tmem_o + map * TD + t_lane + c0, orr);
+          tmem_ld_32x32(tmem_o + (map + group) * TD + t_lane + c0, orr);
           tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 32; ++j) orr[j] = __float_as_uint(__uint_as_float(orr[j]) * alpha);
-          tmem_st_32x32(tmem_o + map * TD + t_lane + c0, orr);
+          tmem_st_32x32(tmem_o + (map + group) * TD + t_lane + c0, orr);
         }
         tmem_st_wait();
       }
       fence_proxy_async();          // P (generic-proxy stores) -> visible to the MMA's async-proxy reads
       tc_fence_before();
-      mbar_arrive(&p_full[2 * map + sb]);
+      mbar_arrive(&p_full[buf]);
       if (tid == 0 && i < 8) attn_trace(24 + i);   // P of tile i published
     }
     // ---- epilogue
-    if (ok) ok = mbar_wait_backoff(o_done, 0, p.status, kTimeoutAccum);
+    if (ok) ok = attn_wait<TMA>(o_done, 0, p.status, kTimeoutAccum);
     tc_fence_after();
     if (tid == 0) attn_trace(3);    // output accumulator complete
     sm_ok = ok;
@@ -601,6 +734,50 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
         uint4* dst = reinterpret_cast<uint4*>(out_ptr + map * 64);
 #pragma unroll
         for (int j = 0; j < 8; ++j) dst[j] = pk[j];
+      }
+    } else if constexpr (MODE == kTwo) {
+      // both groups' threads of a row finish half of its columns each; maxima and sums pass through the dead Q tile
+      float2* ml2 = reinterpret_cast<float2*>(sQ);
+      ml2[group * TROWS + row] = make_float2(m_run, l_run);
+      const bool both_ok = named_and(ok, 2 * TROWS);
+      const float2 a = ml2[row], c = ml2[TROWS + row];
+      const float m = fmaxf(a.x, c.x), m_safe = m == -INFINITY ? 0.f : m;
+      // a group that saw no key of this row (sum 0) does not count; with a single tile it has no accumulator either
+      const bool has0 = a.y != 0.f, has1 = c.y != 0.f;
+      const float w0 = exp2f(a.x - m_safe), w1 = exp2f(c.x - m_safe);
+      const float l = (has0 ? a.y * w0 : 0.f) + (has1 ? c.y * w1 : 0.f);
+      const float f = p.splits > 1 ? 1.f : l > 0.f ? gate / l : 0.f;
+      if (both_ok) {
+#pragma unroll 1
+        for (int c0 = group * 64; c0 < group * 64 + 64; c0 += 32) {
+          uint32_t u[32], v[32];
+          tmem_ld_32x32(tmem_o + t_lane + c0, u);
+          tmem_ld_32x32(tmem_o + TD + t_lane + c0, v);
+          tmem_ld_wait();
+          if (!row_valid) continue;
+          float o[32];
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            o[j] = ((has0 ? __uint_as_float(u[j]) * w0 : 0.f) + (has1 ? __uint_as_float(v[j]) * w1 : 0.f)) * f;
+          if (p.splits == 1) {
+            uint4 pk[4];
+            __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(pk);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) o2[j] = __floats2bfloat162_rn(o[2 * j], o[2 * j + 1]);
+            uint4* dst = reinterpret_cast<uint4*>(out_ptr + c0);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) dst[j] = pk[j];
+          } else {
+            float4* dst = reinterpret_cast<float4*>(p.ws_o + (static_cast<size_t>(split) * p.T * p.Hq + out_row) * TD + c0);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) dst[j] = make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+          }
+        }
+        if (p.splits > 1 && row_valid && group == 0) {
+          float* ml = p.ws_ml + (static_cast<size_t>(split) * p.T * p.Hq + out_row) * 2;
+          ml[0] = m;
+          ml[1] = l;
+        }
       }
     } else if (ok && !cmerge) {
       const float inv = l_run > 0.f ? gate / l_run : 0.f;
@@ -712,7 +889,7 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
   __syncthreads();
   if (warp == MMA_WARP && nt > 0) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 256 * MAPS);
+    tmem_dealloc(tmem_base, 256 * GROUPS);
   }
 }
 
@@ -752,7 +929,7 @@ __global__ void __launch_bounds__(256) diff_merge_kernel(AttnTcParams p) {
 }
 
 template <int G, int MODE>
-static int launch_attn_tc(const AttnTcParams& p, int q_tiles, bool pdl, cudaStream_t stream) {
+static int launch_attn_tc(const AttnTcParams& p, const AttnMaps& maps, int q_tiles, bool pdl, cudaStream_t stream) {
   static int configured[kMaxDevicesCached] = {};
   constexpr int kAttnTcSmem = attn_tc_smem(MODE);
   auto kern = paged_tree_attn_tc_kernel<G, MODE>;
@@ -778,7 +955,26 @@ static int launch_attn_tc(const AttnTcParams& p, int q_tiles, bool pdl, cudaStre
   }
   cfg.attrs = attr;
   cfg.numAttrs = na;
-  return cudaLaunchKernelEx(&cfg, kern, p) == cudaSuccess ? 0 : -4;
+  return cudaLaunchKernelEx(&cfg, kern, p, maps) == cudaSuccess ? 0 : -4;
+}
+
+// Tensor maps of the pools, or false for a layout that no such map describes.
+static bool make_attn_maps(AttnMaps* m, const void* k, const void* v, int Hkv, int S, long long kv_head, long long kv_slot) {
+  uint64_t rows = S, cols = TD;
+  m->head_rows = m->head_cols = 0;
+  if (Hkv > 1) {
+    if (kv_head >= kv_slot && kv_head % kv_slot == 0) {        // a head's slots are whole rows further on
+      m->head_rows = static_cast<int>(kv_head / kv_slot);
+      rows += static_cast<uint64_t>(Hkv - 1) * m->head_rows;
+    } else if (kv_head > 0 && (Hkv - 1) * kv_head + TD <= kv_slot) {   // heads side by side in a slot's row
+      m->head_cols = static_cast<int>(kv_head);
+      cols += static_cast<uint64_t>(Hkv - 1) * kv_head;
+    } else {
+      return false;
+    }
+  }
+  return kv_slot >= TD && rows < (1ull << 31) && !make_map(&m->k16, k, rows, cols, kv_slot, 16) && !make_map(&m->v16, v, rows, cols, kv_slot, 16) &&
+         !make_map(&m->k1, k, rows, cols, kv_slot, 1) && !make_map(&m->v1, v, rows, cols, kv_slot, 1);
 }
 
 }  // namespace js
@@ -869,6 +1065,9 @@ extern "C" int js_window_attention_tc(const void* q, const void* k_pool, const v
     const int npt = 128 / G;
     in_cluster = r > 0 && ((T + npt - 1) / npt) * Hkv <= r;
   }
+  // Two softmax groups where a CTA has many tiles: without splits (many query rows), or with long ones.  A decode round's
+  // splits hold a few tiles each, and merging in the cluster counts for more there.
+  const bool two = splits == 1 || (!in_cluster && max_len >= 1024 * splits);
   AttnTcParams p{reinterpret_cast<const __nv_bfloat16*>(q), reinterpret_cast<const __nv_bfloat16*>(k_pool),
                  reinterpret_cast<const __nv_bfloat16*>(v_pool), slot_map, seq_rows, cu_q, past_lens, mask_bits,
                  reinterpret_cast<__nv_bfloat16*>(out), ws_o, ws_ml, status, B, T, Hq, Hkv, S, max_len, W, causal,
@@ -876,19 +1075,23 @@ extern "C" int js_window_attention_tc(const void* q, const void* k_pool, const v
                  in_cluster ? 1 : 0, softcap * 1.4426950408889634f, softcap > 0.f ? 2.8853900817779268f * scale / softcap : 0.f, P,
                  reinterpret_cast<const __nv_bfloat16*>(kb), reinterpret_cast<const __nv_bfloat16*>(vb), block_map, block_rows, max_blocks,
                  lam, share, eps, V};
+  // A layout without tensor maps takes the cp.async form, which is kPlain when there are no blocks and no cap.
+  AttnMaps tm;
+  const bool gathered = maps == 1 && P == 0 && softcap <= 0.f && make_attn_maps(&tm, k_pool, v_pool, Hkv, S, kv_head, kv_slot);
   auto launch = [&](auto mode) {
     constexpr int M = decltype(mode)::value;
     switch (G) {
-      case 1: return launch_attn_tc<1, M>(p, (T + 127) / 128 + B, pdl != 0, stream);
-      case 2: return launch_attn_tc<2, M>(p, (T + 63) / 64 + B, pdl != 0, stream);
-      case 4: return launch_attn_tc<4, M>(p, (T + 31) / 32 + B, pdl != 0, stream);
-      case 8: return launch_attn_tc<8, M>(p, (T + 15) / 16 + B, pdl != 0, stream);
-      case 16: return launch_attn_tc<16, M>(p, (T + 7) / 8 + B, pdl != 0, stream);
+      case 1: return launch_attn_tc<1, M>(p, tm, (T + 127) / 128 + B, pdl != 0, stream);
+      case 2: return launch_attn_tc<2, M>(p, tm, (T + 63) / 64 + B, pdl != 0, stream);
+      case 4: return launch_attn_tc<4, M>(p, tm, (T + 31) / 32 + B, pdl != 0, stream);
+      case 8: return launch_attn_tc<8, M>(p, tm, (T + 15) / 16 + B, pdl != 0, stream);
+      case 16: return launch_attn_tc<16, M>(p, tm, (T + 7) / 8 + B, pdl != 0, stream);
       default: return -14;
     }
   };
   const int rc = maps == 2 ? launch(std::integral_constant<int, kDiff>{})
-               : P > 0 || softcap > 0.f ? launch(std::integral_constant<int, kPooled>{}) : launch(std::integral_constant<int, kPlain>{});
+               : !gathered ? launch(std::integral_constant<int, kPooled>{})
+               : two ? launch(std::integral_constant<int, kTwo>{}) : launch(std::integral_constant<int, kPlain>{});
   if (rc != 0 || splits == 1 || p.cluster_merge) return rc;
   if (maps == 1) return js_attn_merge(ws_o, ws_ml, gate, ldg, out, ldo, T, Hq, splits, pdl, stream);
   cudaLaunchConfig_t c2 = {};

@@ -633,7 +633,7 @@ def paged_tree_attention(q, k_pool, v_pool, slot_map, seq_rows, cu_q, past_lens,
         out = torch.empty(T, Hq * D, dtype=q.dtype, device=q.device)
     if splits is None:
         mk = max_keys if max_keys is not None else slot_map.shape[1]
-        splits = attn_splits_for(T, Hq, Hkv, mk)
+        splits = attn_splits_for(T, Hq, Hkv, mk, B)
     ws_o = ws_ml = None
     if splits > 1:
         if ws is None:

@@ -324,6 +324,36 @@ def test_paged_tree_attention(ext, Hq, Hkv, splits, causal, impl):
     ext.check_status("cuda")
 
 
+@pytest.mark.parametrize("Hq,Hkv,splits,causal", [(32, 8, 1, False), (32, 8, 1, True), (8, 8, 2, False), (8, 8, 3, True), (16, 1, 1, False)])
+def test_paged_attention_of_two_softmax_groups(ext, Hq, Hkv, splits, causal):
+    """Key tiles taken in turn by two groups: sequences of 1, 2, 3, 4, 5, 8 and 9 tiles and of a length between, a group without a
+    tile, rows that see keys of one group only, long splits that leave partial results to the merge."""
+    from jetspec_b200.ops import reference as ref
+    rng = random.Random(11)
+    pasts, ns = [0, 64, 180, 250, 319, 511, 512, 60, 1900], [1, 3, 9, 6, 1, 1, 64, 130, 9]
+    if splits > 1:
+        ns[7], ns[6] = 1000 if causal else 250, 900 if causal else 256
+        ns[5] = ns[4] = 256
+        ns[8] = 120                                # enough rows that the splits do not form resident clusters
+    B, T, S, max_len = len(ns), sum(ns), 8192, 3072
+    kp, vp, q = rnd(Hkv, S, 128, seed=32), rnd(Hkv, S, 128, seed=33), rnd(T, Hq, 128, seed=34)
+    perm = torch.randperm(S, device="cuda").to(torch.int32)
+    slot_map, off = torch.zeros(B, max_len, dtype=torch.int32, device="cuda"), 0
+    for b in range(B):
+        slot_map[b, :pasts[b] + ns[b]] = perm[off:off + pasts[b] + ns[b]]
+        off += pasts[b] + ns[b]
+    cu = torch.tensor([0] + torch.tensor(ns).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+    bits = None if causal else torch.cat([_random_tree_bits(n, 8, rng) for n in ns]).cuda()
+    seq_rows, past = torch.arange(B, dtype=torch.int32, device="cuda"), torch.tensor(pasts, dtype=torch.int32, device="cuda")
+    out = ext.paged_tree_attention(q, kp, vp, slot_map, seq_rows, cu, past, bits, 0.1, causal, max(ns), splits=splits, impl="tc")
+    want = ref.paged_tree_attention(q.float(), kp.float(), vp.float(), slot_map, seq_rows, cu, past, bits, 0.1, causal)
+    assert rel_err(out, want) < BF16_TOL
+    q[0] = float("nan")                            # the first sequence's only row: one tile, one group
+    out = ext.paged_tree_attention(q, kp, vp, slot_map, seq_rows, cu, past, bits, 0.1, causal, max(ns), splits=splits, impl="tc")
+    assert torch.isnan(out[0]).all() and rel_err(out[1:], want[1:]) < BF16_TOL
+    ext.check_status("cuda")
+
+
 @pytest.mark.parametrize("seed", range(4))
 def test_device_tree_build_and_accept_match_host(ext, seed):
     import ctypes
