@@ -61,9 +61,16 @@ JS_DEVICE unsigned long long gtime() {
 // one CTA per SM a deeper pipeline.
 // MT = row tiles per CTA (1 or 2): with 2, one CTA computes a 256 x BN tile as two 128-row accumulators that share
 // every weight stage, so a k-block brings 1.5x the FLOPs per byte through the L2-to-SM path (many-row GEMMs).
-template <int BN, int BUDGET_KB, bool FP4 = false, int MT = 1>
+// AR = activation rows a stage holds (16, 32 or all 128), for launches of one row tile with at most that many rows: the MMA
+// still reads 128 rows from the start of a stage's activations and meets the stage's weights behind them, which only
+// touches accumulator rows that are never stored.  At AR = 16 a stage is 18 KB instead of 32, so that 96 KB keep five weight
+// tiles in flight instead of three, and the K-split exchange carries AR rows instead of 128.  One row (us a launch, before /
+// after): 24576 x 4096 40.1 / 37.9, 4096 x 12288 21.7 / 19.9, 4096 x 4096 11.4 / 10.2, 6144 x 4096 14.0 / 13.8; plain decode of
+// Qwen3-8B sizes 66.0 / 62.5 ms for 16 tokens.  More than eight stages, or every launch at 96 KB, measured no better there.
+template <int BN, int BUDGET_KB, bool FP4 = false, int MT = 1, int AR = BM>
 struct GemmSmem {
-  static constexpr int kStageA = MT * BM * BK * 2; // 128-byte rows in both modes
+  static_assert(AR == BM || (BN >= 128 && MT == 1 && AR % 8 == 0), "the weights of a stage cover what the MMA reads");
+  static constexpr int kStageA = MT * AR * BK * 2; // 128-byte rows in both modes
   static constexpr int kStageW = BN * BK * 2;
   static constexpr int kStageSF = FP4 ? 2048 + (BN / 128) * 2048 : 0;   // 4 scale tiles of A + 4 per 128 rows of W
   static constexpr int kStage = kStageA + kStageW + kStageSF;
@@ -81,8 +88,8 @@ __host__ __device__ inline int recv_slots_per_src(int split, int bn, bool swiglu
   const int per = (hc + split - 1) / split;
   return swiglu ? 2 * per : per;
 }
-__host__ __device__ inline int recv_bytes(int split, int bn, bool swiglu) {
-  return split > 1 ? split * recv_slots_per_src(split, bn, swiglu) * 16384 : 0;
+__host__ __device__ inline int recv_bytes(int split, int bn, bool swiglu, int rows = BM) {
+  return split > 1 ? split * recv_slots_per_src(split, bn, swiglu) * (32 * 4 * rows) : 0;
 }
 
 // The receive area shares the stages' memory only when the two do not fit side by side.
@@ -90,11 +97,12 @@ __host__ __device__ inline bool recv_aliases_stages(int tiles_bytes, int recv_to
   return recv_total > 0 && tiles_bytes + recv_total + 1280 > 227 * 1024;
 }
 
-template <int BN, int EPI, int BUDGET_KB, bool FP4 = false, int MT = 1>
-__global__ void __launch_bounds__(kGemmThreads, GemmSmem<BN, BUDGET_KB, FP4, MT>::kMinBlocks)
+template <int BN, int EPI, int BUDGET_KB, bool FP4 = false, int MT = 1, int AR = BM>
+__global__ void __launch_bounds__(kGemmThreads, GemmSmem<BN, BUDGET_KB, FP4, MT, AR>::kMinBlocks)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW,
                  const __grid_constant__ CUtensorMap tmA2, GemmParams p) {
-  using S = GemmSmem<BN, BUDGET_KB, FP4, MT>;
+  using S = GemmSmem<BN, BUDGET_KB, FP4, MT, AR>;
+  static_assert(AR == BM || (EPI != EPI_TOPK && EPI != EPI_ALLREDUCE && EPI != EPI_EP_COMBINE), "all epilogue warps take part");
   constexpr int kStages = S::kStages;
   static_assert(!FP4 || BN == 128, "the NVFP4 path is built for 128-column tiles");
   static_assert(MT == 1 || (MT == 2 && !FP4 && BN == 256), "two row tiles per CTA: bf16, 256-column tiles, no K split");
@@ -111,7 +119,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   // not fit (deep pipeline) it ALIASES them, guarded by one more cluster barrier after the main loop.
   const bool grouped = p.group_off != nullptr;
   const bool zbatch = grouped || p.batch > 0;     // blockIdx.z counts experts or batch elements, not K splits
-  const int recv_total = recv_bytes(zbatch ? 1 : gridDim.z, BN, EPI == EPI_SWIGLU || EPI == EPI_INPROJ);
+  const int recv_total = recv_bytes(zbatch ? 1 : gridDim.z, BN, EPI == EPI_SWIGLU || EPI == EPI_INPROJ, AR);
   const bool alias = recv_aliases_stages(S::kTiles, recv_total);
   const int data_bytes = alias ? (S::kTiles > recv_total ? S::kTiles : recv_total) : S::kTiles + recv_total;
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + data_bytes);
@@ -303,7 +311,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 
   // ------------------------------------------------------------------ epilogue
-  const bool epi_warp = warp >= 2;
+  const bool epi_warp = warp >= 2 && (AR == BM || (warp & 3) * 32 < AR);     // warps whose rows are never valid sit out
   const int quad = warp & 3;                     // TMEM lane quadrant this warp may read
   const int row = quad * 32 + lane;              // row of the tile owned by this thread
   uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
@@ -347,9 +355,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         tmem_ld_32x32(t_row + ch * 32, r);
         tmem_ld_wait();
         const uint32_t dst = map_to_cta(recv_addr, owner_of(ch)) +
-                             static_cast<uint32_t>((z * slots_per_src + local_of(ch)) * 16384 + row * 4);
+                             static_cast<uint32_t>((z * slots_per_src + local_of(ch)) * (32 * 4 * AR) + row * 4);
+        if (AR >= 32 || lane < AR) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) st_dsmem_f32(dst + j * (BM * 4), __uint_as_float(r[j]));
+          for (int j = 0; j < 32; ++j) st_dsmem_f32(dst + j * (AR * 4), __uint_as_float(r[j]));
+        }
+        __syncwarp();
       }
     }
     tc_fence_before();
@@ -378,9 +389,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         for (int j = 0; j < 32; ++j) v[j] = 0.f;
         const int lo = local_of(c0 >> 5);
         for (int src = 0; src < split; ++src) {   // fixed source order: deterministic sum
-          const float* base = recv + (src * slots_per_src + lo) * 4096 + row;
+          const float* base = recv + (src * slots_per_src + lo) * (32 * AR) + (AR < 32 ? row & (AR - 1) : row);
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] += base[j * BM];
+          for (int j = 0; j < 32; ++j) v[j] += base[j * AR];
         }
       }
       if constexpr (FP4) {
@@ -821,14 +832,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
 // ---------------------------------------------------------------------------- host side
 constexpr int kGroupedSmallRows = 32;     // rows of the small activation box of grouped launches (GemmParams::a_small_rows)
-template <int BN, int EPI, int BUDGET_KB, bool FP4 = false, int MT = 1>
+template <int BN, int EPI, int BUDGET_KB, bool FP4 = false, int MT = 1, int AR = BM>
 static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tw, const GemmParams& p, int split, bool pdl,
                        cudaStream_t stream, int groups = 0, int group_m_tiles = 0, const CUtensorMap* ta_small = nullptr) {
-  using S = GemmSmem<BN, BUDGET_KB, FP4, MT>;
+  using S = GemmSmem<BN, BUDGET_KB, FP4, MT, AR>;
   static int configured[kMaxDevicesCached] = {};
-  auto kern = gemm_bf16_kernel<BN, EPI, BUDGET_KB, FP4, MT>;
+  auto kern = gemm_bf16_kernel<BN, EPI, BUDGET_KB, FP4, MT, AR>;
+  if (AR != BM && (p.M > AR || groups > 0)) return -19;
   if (MT != 1 && (split != 1 || groups > 0)) return -19;
-  const int recv_total = recv_bytes(split, BN, EPI == EPI_SWIGLU || EPI == EPI_INPROJ);
+  const int recv_total = recv_bytes(split, BN, EPI == EPI_SWIGLU || EPI == EPI_INPROJ, AR);
   const int data_bytes = recv_aliases_stages(S::kTiles, recv_total) ? (S::kTiles > recv_total ? S::kTiles : recv_total)
                                                                      : S::kTiles + recv_total;
   const int smem_bytes = data_bytes + 1024 /*align slack*/ + 256 /*barriers*/ + ((EPI == EPI_ALLREDUCE || EPI == EPI_EP_COMBINE) ? 8192 + 64 : 0);
@@ -856,10 +868,19 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tw, const GemmP
   cfg.numAttrs = na;
   return cudaLaunchKernelEx(&cfg, kern, ta, tw, ta_small ? *ta_small : ta, p) == cudaSuccess ? 0 : -4;
 }
-template <int BN, int EPI, int BUDGET_KB, bool FP4 = false, int MT = 1>
+template <int BN, int EPI, int BUDGET_KB, bool FP4 = false, int MT = 1, int AR = BM>
 static int launch_gemm(const ActMaps& ta, const CUtensorMap& tw, const GemmParams& p, int split, bool pdl, cudaStream_t stream) {
-  return launch_gemm<BN, EPI, BUDGET_KB, FP4, MT>(ta.full, tw, p, split, pdl, stream, 0, 0,
+  return launch_gemm<BN, EPI, BUDGET_KB, FP4, MT, AR>(ta.full, tw, p, split, pdl, stream, 0, 0,
                                                   p.a_small_rows > 0 ? &ta.last : nullptr);
+}
+// Launches of at most 32 rows on 128-column tiles; deep as in js_gemm_bf16 (0, 2: 96 KB, 1: eight stages)
+template <int EPI>
+static int launch_few_rows(const ActMaps& ta, const CUtensorMap& tw, const GemmParams& p, int split, int deep, bool pdl, cudaStream_t stream) {
+  if (p.M <= 16)
+    return deep == 1 ? launch_gemm<128, EPI, 192, false, 1, 16>(ta, tw, p, split, pdl, stream)
+                     : launch_gemm<128, EPI, 96, false, 1, 16>(ta, tw, p, split, pdl, stream);
+  return deep == 1 ? launch_gemm<128, EPI, 192, false, 1, 32>(ta, tw, p, split, pdl, stream)
+                   : launch_gemm<128, EPI, 96, false, 1, 32>(ta, tw, p, split, pdl, stream);
 }
 
 }  // namespace js
@@ -896,6 +917,12 @@ extern "C" int js_gemm_bf16(const void* A, const void* W, void* C, const void* r
     if (epi == EPI_STORE) return launch_gemm<256, EPI_STORE, 192, false, 2>(ta, tw, p, 1, pdl != 0, stream);
     if (epi == EPI_SWIGLU) return launch_gemm<256, EPI_SWIGLU, 192, false, 2>(ta, tw, p, 1, pdl != 0, stream);
     return -19;
+  }
+  if (bn == 128 && M <= 32) {
+    if (epi == EPI_STORE) return launch_few_rows<EPI_STORE>(ta, tw, p, split, deep, pdl != 0, stream);
+    if (epi == EPI_STORE_F32) return launch_few_rows<EPI_STORE_F32>(ta, tw, p, split, deep, pdl != 0, stream);
+    if (epi == EPI_SWIGLU) return launch_few_rows<EPI_SWIGLU>(ta, tw, p, split, deep, pdl != 0, stream);
+    if (epi == EPI_ARGMAX) return launch_few_rows<EPI_ARGMAX>(ta, tw, p, split, deep, pdl != 0, stream);
   }
 #define JS_CASE(BN_, EPI_)                                                                              \
   if (bn == BN_ && epi == EPI_)                                                                         \
@@ -1093,6 +1120,7 @@ extern "C" int js_gemm_inproj(const void* A, const void* W, float* C, void* C2, 
   ActMaps ta;
   CUtensorMap tw;
   if (make_act_maps(&ta, &p, A, K, lda, false) || make_map(&tw, W, N, K, ldw, bn)) return -16;
+  if (bn == 128 && M <= 32) return launch_few_rows<EPI_INPROJ>(ta, tw, p, split, deep, pdl != 0, stream);
   if (bn == 128)
     return deep == 1   ? launch_gemm<128, EPI_INPROJ, 192>(ta, tw, p, split, pdl != 0, stream)
            : deep == 2 ? launch_gemm<128, EPI_INPROJ, 128>(ta, tw, p, split, pdl != 0, stream)
@@ -1121,6 +1149,7 @@ extern "C" int js_gemm_resid32(const void* A, const void* W, float* x_out, const
   ActMaps ta;
   CUtensorMap tw;
   if (make_act_maps(&ta, &p, A, K, lda, false) || make_map(&tw, W, N, K, ldw, bn)) return -16;
+  if (bn == 128 && M <= 32) return launch_few_rows<EPI_RESID32>(ta, tw, p, split, deep, pdl != 0, stream);
   if (bn == 128)
     return deep == 1   ? launch_gemm<128, EPI_RESID32, 192>(ta, tw, p, split, pdl != 0, stream)
            : deep == 2 ? launch_gemm<128, EPI_RESID32, 128>(ta, tw, p, split, pdl != 0, stream)

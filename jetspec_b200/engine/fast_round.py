@@ -108,9 +108,8 @@ def _finish_layer_weights(out: list) -> list:
     return out
 
 
-# Rows of a prefill portion: wide enough that its GEMMs are bound by the tensor cores (512-row portions took 277 us a
-# layer of Qwen3-8B's GEMMs, 4 x 277 for the rows that one 2048-row portion takes in 675), few enough that the
-# activations stay in the tens of megabytes.
+# Rows of a prefill portion: wide enough that its GEMMs are bound by the tensor cores (a layer of Qwen3-8B's: 537 us for one
+# portion of 2048 rows, 4 x 171 for four of 512), few enough that the activations stay in the tens of megabytes.
 _PREFILL_ROWS = 2048
 
 

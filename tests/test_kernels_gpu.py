@@ -163,6 +163,30 @@ def test_inproj_and_resid32_on_cta_pairs(ext, M, monkeypatch):
     ext.check_status("cuda")
 
 
+@pytest.mark.parametrize("M", [1, 15, 16, 17, 31, 32, 33])
+@pytest.mark.parametrize("split", [1, 2, 3, 4])
+def test_gemm_few_rows(ext, M, split):
+    """Stages and K-split exchange of 16 and of 32 activation rows, and the first row count past them; both pipeline depths."""
+    K, N = 1000, 768
+    pad, w = rnd(M + 3, K, seed=70), rnd(N, K, scale=0.05, seed=71)
+    pad[M:] = float("nan")
+    x, r = pad[:M], rnd(M, N, seed=72)
+    ref = x.float() @ w.float().t()
+    wi = ext.interleave_gate_up(w[:N // 2], w[N // 2:])
+    for deep in (0, 1):
+        kw = dict(bn=128, split=split, deep=deep)
+        assert rel_err(ext.gemm(x, w, residual=r, **kw), ref + r.float()) < BF16_TOL
+        assert rel_err(ext.gemm(x, w, epi=ext.EPI_STORE_F32, **kw), ref) < 1e-4
+        assert rel_err(ext.gemm(x, wi, epi=ext.EPI_SWIGLU, **kw), torch.nn.functional.silu(ref[:, :384]) * ref[:, 384:]) < BF16_TOL
+        raw, act = torch.empty(M, 256, device="cuda"), torch.empty(M, 512, dtype=torch.bfloat16, device="cuda")
+        ext.gemm_inproj(x, w, raw, 256, act, False, act=ext.ACT_GELU_ERF, **kw)
+        assert rel_err(raw, ref[:, :256]) < 1e-4 and rel_err(act, torch.nn.functional.gelu(ref[:, 256:])) < BF16_TOL
+        y = torch.ones(M, N, device="cuda")
+        ext.gemm_resid32(x, w, y, **kw)
+        assert rel_err(y, ref + 1) < 1e-4
+    ext.check_status("cuda")
+
+
 def test_gemm_fp32_out(ext):
     x, w = rnd(64, 512, seed=6), rnd(128, 512, scale=0.05, seed=7)
     out = ext.gemm(x, w, epi=ext.EPI_STORE_F32, split=2)
