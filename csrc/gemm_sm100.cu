@@ -178,6 +178,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // Waited for before the first store to a peer, which must have started by then (the aliased form joins its own barrier
+  // behind the main loop).
+  if (split > 1 && !alias) cluster_arrive();
 
   // Let the next kernel in the stream start its own prologue; it still waits for this grid
   // to finish before touching our output.
@@ -341,7 +344,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 
   if (split > 1) {
-    if (alias) {   // every CTA of the cluster has finished its main loop (its stages are dead) before anyone pushes
+    __syncwarp();
+    if (!alias) {
+      cluster_wait();
+    } else {       // every CTA of the cluster has finished its main loop (its stages are dead) before anyone pushes
       tc_fence_before();
       __syncthreads();
       cluster_sync();

@@ -187,6 +187,20 @@ def test_gemm_few_rows(ext, M, split):
     ext.check_status("cuda")
 
 
+@pytest.mark.parametrize("M,deep", [(1, 1), (16, 0), (17, 1), (32, 0), (100, 0), (128, 2)])
+@pytest.mark.parametrize("split", [2, 4])
+def test_gemm_split_pushes_meet_started_peers(ext, M, deep, split):
+    """K-split forms whose receive area lies beside the stages: a CTA may store to a peer before that peer's main loop is over,
+    but not before it runs.  Few k-blocks, so that a CTA is done early; launches back to back, each allowed to start
+    under the one before; the sum's order is fixed, so every launch gives the same bits."""
+    K, N = 256, 4096
+    x, w = rnd(M, K, seed=80), rnd(N, K, scale=0.05, seed=81)
+    outs = [ext.gemm(x, w, bn=128, split=split, deep=deep, pdl=True) for _ in range(40)]
+    assert rel_err(outs[0], x.float() @ w.float().t()) < BF16_TOL
+    assert all(torch.equal(o, outs[0]) for o in outs)
+    ext.check_status("cuda")
+
+
 def test_gemm_fp32_out(ext):
     x, w = rnd(64, 512, seed=6), rnd(128, 512, scale=0.05, seed=7)
     out = ext.gemm(x, w, epi=ext.EPI_STORE_F32, split=2)
