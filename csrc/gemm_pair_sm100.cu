@@ -158,6 +158,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (++s == kPairStages) { s = 0; phase ^= 1; }
       }
     }
+    // Every commit that frees a stage arrives here as well as in the other CTA: a CTA stays until the last of them has
+    // landed, and with them its loads (a stage that was never filled counts as free).
+    for (int i = 0; i < kPairStages && ok; ++i) {
+      ok = mbar_wait(&empty_bar[s], phase, p.status, kTimeoutEmpty);
+      if (++s == kPairStages) { s = 0; phase ^= 1; }
+    }
   } else if (warp == 1) {
     if (rank == 0) {
       constexpr uint32_t idesc = umma_idesc_bf16(kPairRows, TN);
@@ -272,7 +278,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   }
 
-  // Nobody leaves while the pair's MMAs may still read its shared memory or its arrivals may still land there.
+  // Nobody leaves while the pair's MMAs may still read its shared memory or an arrival may still land there: the commits
+  // were waited for above, the other CTA's arrivals on accum_free come before it joins this barrier.
   tc_fence_before();
   __syncthreads();
   cluster_sync();

@@ -135,6 +135,20 @@ def test_gemm_on_cta_pairs(ext, M, N, K):
     ext.check_status("cuda")
 
 
+@pytest.mark.parametrize("K", [64, 320, 640])
+@pytest.mark.parametrize("tile", [128, 256])
+def test_cta_pairs_leave_after_their_last_commit(ext, K, tile):
+    """Fewer k-blocks than stages, as many and more: the stages of a pair's last k-blocks are freed in both CTAs while the
+    first may already be at its end.  Launches back to back, each allowed to start under the one before, take over the SMs
+    (and the barriers' shared memory) of CTAs that just left; every launch gives the same bits."""
+    M, N = 300, 4096
+    x, w = rnd(M, K, seed=82), rnd(N, K, scale=0.05, seed=83)
+    outs = [ext.gemm(x, w, pair=tile, pdl=True) for _ in range(40)]
+    assert rel_err(outs[0], x.float() @ w.float().t()) < BF16_TOL
+    assert all(torch.equal(o, outs[0]) for o in outs)
+    ext.check_status("cuda")
+
+
 @pytest.mark.parametrize("M", [200, 640])
 def test_inproj_and_resid32_on_cta_pairs(ext, M, monkeypatch):
     K, N, n_raw = 192, 768, 256
