@@ -71,6 +71,14 @@ JS_DEVICE bool lat_mbar_wait(uint64_t* bar, uint32_t parity, int* status, int co
   report(status, code);
   return false;
 }
+// of a whole warp with warp-wide steps to come
+JS_DEVICE bool lat_warp_wait(uint64_t* bar, uint32_t parity, int* status, int code, uint32_t* gave_up) {
+  for (uint32_t i = 0;; ++i) {
+    if (mbar_test_wait(bar, parity)) return true;
+    if (i >= (kSpinLimit >> 2) && warp_gives_up(bar, parity, status, code, gave_up)) return false;
+    __nanosleep(20);
+  }
+}
 JS_DEVICE float lat_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -122,6 +130,7 @@ __global__ void __launch_bounds__(LTHREADS, 1) latent_attn_tc_kernel(LatentAttnP
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  uint32_t* gave_up = tmem_slot + 1 + (warp & 3);       // of a softmax warp
   const int grp = blockIdx.y, split = blockIdx.z;
   const int v0 = grp == 0 ? 0 : p.chunks0;                       // first column chunk of this CTA's output
   const int nv = grp == 0 ? p.chunks0 : p.nout - p.chunks0;      // and how many (at most 4)
@@ -169,6 +178,7 @@ __global__ void __launch_bounds__(LTHREADS, 1) latent_attn_tc_kernel(LatentAttnP
     for (int s = 0; s < NST; ++s) { mbar_init(&kv_full[s], LLOADERS); mbar_init(&kv_empty[s], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 128); mbar_init(&pv_done[i], 1); }
     mbar_init(o_done, 1);
+    for (int w = 0; w < 4; ++w) tmem_slot[1 + w] = 0;
     fence_barrier_init();
   }
   const uint32_t tmem_cols = nv > 2 ? 512u : 256u;
@@ -320,7 +330,7 @@ __global__ void __launch_bounds__(LTHREADS, 1) latent_attn_tc_kernel(LatentAttnP
     bool ok = true;
     for (int i = 0; i < nt && ok; ++i) {
       const int sb = i & 1;
-      ok = lat_mbar_wait(&s_full[sb], (i >> 1) & 1, p.status, kTimeoutAccum);
+      ok = lat_warp_wait(&s_full[sb], (i >> 1) & 1, p.status, kTimeoutAccum, gave_up);
       if (!ok) break;
       tc_fence_after();
       uint32_t sr[TK];
@@ -374,7 +384,7 @@ __global__ void __launch_bounds__(LTHREADS, 1) latent_attn_tc_kernel(LatentAttnP
       const float alpha = exp2f(m_run - m_safe);
       const bool need = i > 0 && m_run != -INFINITY && alpha != 1.f;   // nothing accumulated yet: nothing to rescale
       m_run = m_new;
-      if (i >= 2) ok = lat_mbar_wait(&pv_done[sb], ((i - 2) >> 1) & 1, p.status, kTimeoutAccum);
+      if (i >= 2) ok = lat_warp_wait(&pv_done[sb], ((i - 2) >> 1) & 1, p.status, kTimeoutAccum, gave_up);
       if (!ok) break;
       float rs4[4] = {0.f, 0.f, 0.f, 0.f};
       const uint32_t p_row = smem_u32(sP) + (TK == 64 ? sb * RQ * 128 : 0) + row * 128;
@@ -397,7 +407,7 @@ __global__ void __launch_bounds__(LTHREADS, 1) latent_attn_tc_kernel(LatentAttnP
       }
       l_run = l_run * alpha + ((rs4[0] + rs4[1]) + (rs4[2] + rs4[3]));
       if (__any_sync(0xffffffffu, need)) {
-        ok = lat_mbar_wait(&pv_done[(i - 1) & 1], ((i - 1) >> 1) & 1, p.status, kTimeoutAccum);
+        ok = lat_warp_wait(&pv_done[(i - 1) & 1], ((i - 1) >> 1) & 1, p.status, kTimeoutAccum, gave_up);
         if (!ok) break;
         tc_fence_after();
         const float f = need ? alpha : 1.f;
@@ -417,7 +427,7 @@ __global__ void __launch_bounds__(LTHREADS, 1) latent_attn_tc_kernel(LatentAttnP
       mbar_arrive(&p_full[sb]);
     }
     // ---- epilogue
-    if (ok) ok = lat_mbar_wait(o_done, 0, p.status, kTimeoutAccum);
+    if (ok) ok = lat_warp_wait(o_done, 0, p.status, kTimeoutAccum, gave_up);
     tc_fence_after();
     if (ok) {
       float inv = l_run > 0.f ? 1.f / l_run : 0.f;

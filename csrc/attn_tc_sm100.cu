@@ -141,8 +141,8 @@ JS_DEVICE void tmem_st_32x32(uint32_t taddr, const uint32_t* r) {
         "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
       : "memory");
 }
-// Bounded wait that backs off between polls: the waiting roles share the SM's load/store path with the
-// loaders' cp.async traffic, so they must not spin on it.
+// Bounded wait of a thread that backs off between polls (cp.async loaders): the waiting roles share the SM's load/store path
+// with the loaders' cp.async traffic, so they must not spin on it.
 JS_DEVICE bool mbar_wait_backoff(uint64_t* bar, uint32_t parity, int* status, int code) {
   for (uint32_t i = 0; i < (kSpinLimit >> 2); ++i) {
     if (mbar_test_wait(bar, parity)) return true;
@@ -151,10 +151,15 @@ JS_DEVICE bool mbar_wait_backoff(uint64_t* bar, uint32_t parity, int* status, in
   report(status, code);
   return false;
 }
-// The waits of the kernel's roles: without cp.async loaders nothing is disturbed by a suspended try_wait.
+// The waits of the kernel's other roles: without cp.async loaders nothing is disturbed by a suspended try_wait.
 template <bool TMA>
-JS_DEVICE bool attn_wait(uint64_t* bar, uint32_t parity, int* status, int code) {
-  return TMA ? mbar_wait(bar, parity, status, code) : mbar_wait_backoff(bar, parity, status, code);
+JS_DEVICE bool attn_wait(uint64_t* bar, uint32_t parity, int* status, int code, uint32_t* gave_up) {
+  if constexpr (TMA) return mbar_wait_warp(bar, parity, status, code, gave_up);
+  for (uint32_t i = 0;; ++i) {
+    if (mbar_test_wait(bar, parity)) return true;
+    if (i >= (kSpinLimit >> 2) && warp_gives_up(bar, parity, status, code, gave_up)) return false;
+    __nanosleep(20);
+  }
 }
 JS_DEVICE void tma_load_2d_at(uint32_t dst, const CUtensorMap* m, uint64_t* bar, int x, int y) {
   asm volatile(
@@ -241,8 +246,10 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
   uint64_t* pv_done = p_full + NB * MAPS;  // NB a map
   uint64_t* o_done = pv_done + NB * MAPS;  // 1
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 1);
+  static_assert((2 + 2 * TSTAGES + 3 * NB * MAPS) * 8 + 4 + TTHREADS / 32 * 4 <= 256, "barriers and words");
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  uint32_t* gave_up = tmem_slot + 1 + warp;
   const int h = blockIdx.y, split = blockIdx.z;
 
   pdl_launch_dependents();
@@ -325,6 +332,7 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
     for (int s = 0; s < TSTAGES; ++s) { mbar_init(&kv_full[s], TMA ? 4 : TLOADERS); mbar_init(&kv_empty[s], 1); }
     for (int i = 0; i < NB * MAPS; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 128); mbar_init(&pv_done[i], 1); }
     mbar_init(o_done, 1);
+    for (int w = 0; w < TTHREADS / 32; ++w) tmem_slot[1 + w] = 0;
     fence_barrier_init();
   }
   if (warp == MMA_WARP && nt > 0) {
@@ -371,7 +379,7 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
           int slot = next;
           if (i + 1 < nt) next = slot_at(i + 1);
           if (slot < 0 || slot >= p.S) { report(p.status, kBadSlot); slot = 0; }
-          ok = attn_wait<TMA>(&kv_empty[s], phase, p.status, kTimeoutEmpty);
+          ok = attn_wait<TMA>(&kv_empty[s], phase, p.status, kTimeoutEmpty, gave_up);
           if (!ok) break;
           const uint32_t dst = smem_u32(sKV + s * kStageKV) + lw * (16 * 128);
           const int first = __shfl_sync(0xffffffffu, slot, 0);
@@ -445,7 +453,7 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
           // about to block on the consumer: it may itself be waiting for tiles not yet published
           cp_async_wait_tc<0>();
           publish_before(i);
-          ok = attn_wait<TMA>(&kv_empty[s], par, p.status, kTimeoutEmpty);
+          ok = mbar_wait_backoff(&kv_empty[s], par, p.status, kTimeoutEmpty);
         }
       }
       if (!ok) break;
@@ -498,7 +506,7 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
     constexpr uint32_t idesc_pv = umma_idesc_bf16_bmn(TROWS, TD);
     const uint64_t q_desc = umma_desc_sw128(smem_u32(sQ)), k_desc = umma_desc_sw128(smem_u32(sKV)),
                    p_desc = umma_desc_sw128(smem_u32(sP)), v_desc = umma_desc_sw128_mn(smem_u32(sKV) + TKEYS * 256, TKEYS * 128);
-    bool ok = attn_wait<TMA>(q_full, 0, p.status, kTimeoutFull);
+    bool ok = attn_wait<TMA>(q_full, 0, p.status, kTimeoutFull, gave_up);
     if (lane == 0) attn_trace(2);                // Q landed
     // O += P V of tile j for every map, each as soon as its P is there
     auto issue_pv = [&](int j) {
@@ -506,7 +514,7 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
       const uint32_t acc = tmem_o + (MODE == kTwo ? (j & 1) * TD : 0);
 #pragma unroll
       for (int m = 0; m < MAPS; ++m) {
-        if (!attn_wait<TMA>(&p_full[NB * m + pb], (j >> NBSH) & 1, p.status, kTimeoutAccum)) return false;
+        if (!attn_wait<TMA>(&p_full[NB * m + pb], (j >> NBSH) & 1, p.status, kTimeoutAccum, gave_up)) return false;
         tc_fence_after();
         if (elect_one()) {
           const uint64_t a_desc = p_desc + static_cast<uint64_t>((2 * m + (j & 1)) * (kSmemP >> 4));
@@ -523,7 +531,7 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
     };
     for (int i = 0; i < nt && ok; ++i) {
       const int s = i % TSTAGES, sb = i & (NB - 1);
-      ok = attn_wait<TMA>(&kv_full[s], (i / TSTAGES) & 1, p.status, kTimeoutFull);
+      ok = attn_wait<TMA>(&kv_full[s], (i / TSTAGES) & 1, p.status, kTimeoutFull, gave_up);
       if (!ok) break;
       if (lane == 0 && i < 8) attn_trace(8 + i);   // K/V tile i landed
       // S buffer sb was consumed when P of tile i - NB was published (waited for before PV(i - NB), issued at step i - LAG)
@@ -579,7 +587,7 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
     bool ok = true;
     for (int i = group; i < nt && ok; i += LAG) {
       const int sb = i & (NB - 1), buf = NB * map + sb;
-      ok = attn_wait<TMA>(&s_full[buf], (i >> NBSH) & 1, p.status, kTimeoutAccum);
+      ok = attn_wait<TMA>(&s_full[buf], (i >> NBSH) & 1, p.status, kTimeoutAccum, gave_up);
       if (!ok) break;
       tc_fence_after();
       if (tid == 0 && i < 8) attn_trace(16 + i);   // scores of tile i ready
@@ -650,7 +658,7 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
       const float alpha = exp2f(m_run - m_safe);          // 0 when nothing was visible before
       m_run = m_new;
       // the P buffer is free once PV of tile i - 2 has completed
-      if (i >= 2) ok = attn_wait<TMA>(&pv_done[NB * map + ((i - 2) & (NB - 1))], ((i - 2) >> NBSH) & 1, p.status, kTimeoutAccum);
+      if (i >= 2) ok = attn_wait<TMA>(&pv_done[NB * map + ((i - 2) & (NB - 1))], ((i - 2) >> NBSH) & 1, p.status, kTimeoutAccum, gave_up);
       if (!ok) break;
       const uint64_t scale2 = pack_f32x2(to_log2, to_log2), shift2 = pack_f32x2(-m_safe, -m_safe);
       uint64_t rs2[4] = {0ull, 0ull, 0ull, 0ull};         // pairs of partial sums
@@ -677,7 +685,7 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
       // rescale O when some row of this warp raised its maximum (tcgen05.ld/st are warp-wide)
       const bool need = i >= LAG && alpha != 1.f;
       if (__any_sync(0xffffffffu, need)) {
-        ok = attn_wait<TMA>(&pv_done[NB * map + ((i - LAG) & (NB - 1))], ((i - LAG) >> NBSH) & 1, p.status, kTimeoutAccum);   // every earlier PV is in O
+        ok = attn_wait<TMA>(&pv_done[NB * map + ((i - LAG) & (NB - 1))], ((i - LAG) >> NBSH) & 1, p.status, kTimeoutAccum, gave_up);   // every earlier PV is in O
         if (!ok) break;
         tc_fence_after();
 #pragma unroll 1
@@ -697,7 +705,7 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
       if (tid == 0 && i < 8) attn_trace(24 + i);   // P of tile i published
     }
     // ---- epilogue
-    if (ok) ok = attn_wait<TMA>(o_done, 0, p.status, kTimeoutAccum);
+    if (ok) ok = attn_wait<TMA>(o_done, 0, p.status, kTimeoutAccum, gave_up);
     tc_fence_after();
     if (tid == 0) attn_trace(3);    // output accumulator complete
     sm_ok = ok;

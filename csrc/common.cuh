@@ -104,6 +104,36 @@ JS_DEVICE bool mbar_wait(uint64_t* bar, uint32_t parity, int* status, int code) 
   return false;
 }
 
+// The lanes of a warp may run out of polls one by one, and warp-wide steps (elect.sync, tcgen05.ld, shuffles) wait for all
+// 32: in a role with such steps a wait fails for the whole warp or not at all.  Lanes that ran out of polls sign off in
+// `gave_up`, a zeroed word of shared memory that only this warp uses, and go on polling until the word is full, which
+// settles the failure for good, or the signal is there after all and they withdraw.  A lane that saw the signal cannot
+// pass it on (the barrier's next phase needs this warp), so either every lane signs off or every lane sees it.
+// All this lies behind the last poll, in a call of its own that leads back into the polls: a vote per wait, a carried result,
+// a single waiting lane or the same code inline cost 45 cycles a k-block (K-split GEMM of 6144 x 4096 at 1 row: 14.4 us a
+// launch this way, 15.2 those ways; 512 x 4096 x 12288 on 128-column pair tiles 45 and 51), 2 % of a decode step.
+__device__ __noinline__ inline bool warp_gives_up(uint64_t* bar, uint32_t parity, int* status, int code, uint32_t* gave_up) {
+  const uint32_t bit = 1u << (threadIdx.x & 31);
+  atomicOr(gave_up, bit);
+  for (uint32_t i = 0; i < (kSpinLimit << 2); ++i) {      // longer than the other lanes take to run out
+    const uint32_t all = *reinterpret_cast<volatile uint32_t*>(gave_up);
+    if (all == 0xffffffffu) break;
+    if (mbar_test_wait(bar, parity) && atomicCAS(gave_up, all, all & ~bit) == all) return false;
+    __nanosleep(100);
+  }
+  report(status, code);
+  return true;
+}
+// Bounded wait of a warp whose lanes fail together.
+JS_DEVICE bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* status, int code, uint32_t* gave_up) {
+  for (uint32_t i = 0;; ++i) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if (i >= kSpinLimit && warp_gives_up(bar, parity, status, code, gave_up)) return false;
+  }
+}
+// What the lanes say, where the vote is off the critical path.
+JS_DEVICE bool warp_ok(bool ok) { return __all_sync(0xffffffffu, ok); }
+
 // One lane of a converged warp (the same one every time).
 JS_DEVICE bool elect_one() {
   uint32_t pred;

@@ -63,9 +63,9 @@ JS_DEVICE void umma_commit_pair(uint64_t* bar) {
 JS_DEVICE void mbar_arrive_cluster(uint32_t bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// Bounded wait for arrivals of the other CTA too.
-JS_DEVICE bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, int* status, int code) {
-  for (uint32_t i = 0; i < kSpinLimit; ++i) {
+// mbar_wait_warp for arrivals of the other CTA too.
+JS_DEVICE bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, int* status, int code, uint32_t* gave_up) {
+  for (uint32_t i = 0;; ++i) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -73,9 +73,8 @@ JS_DEVICE bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, int* status, in
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     if (ok) return true;
+    if (i >= kSpinLimit && warp_gives_up(bar, parity, status, code, gave_up)) return false;
   }
-  report(status, code);
-  return false;
 }
 
 // HALF (SwiGLU): every 2 HALF weight rows hold HALF gate rows and the HALF up rows of the same outputs
@@ -92,6 +91,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint64_t* accum_full = empty_bar + kPairStages;      // 2
   uint64_t* accum_free = accum_full + 2;               // 2, the first CTA's: 4 epilogue warps of each CTA arrive
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum_free + 2);
+  uint32_t* gave_up = tmem_slot + 2;                   // of the producing and of the issuing warp
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
@@ -112,6 +112,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       mbar_init(&accum_full[b], 1);
       mbar_init(&accum_free[b], 8);
     }
+    gave_up[0] = gave_up[1] = 0;
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -143,7 +144,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const int rows = box_rows(m);
       const uint32_t bytes = static_cast<uint32_t>(2 * kPairHalfW + (box_rows(m0) + box_rows(m0 + BM)) * BK * 2);
       for (int kb = 0; kb < nkb; ++kb) {
-        ok = mbar_wait(&empty_bar[s], phase, p.status, kTimeoutEmpty);
+        ok = mbar_wait_warp(&empty_bar[s], phase, p.status, kTimeoutEmpty, &gave_up[0]);
         if (!ok) break;
         if (elect_one()) {
           // The other CTA's bytes may land before this arrival: it passed its own copy of the empty barrier, so they
@@ -161,7 +162,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // Every commit that frees a stage arrives here as well as in the other CTA: a CTA stays until the last of them has
     // landed, and with them its loads (a stage that was never filled counts as free).
     for (int i = 0; i < kPairStages && ok; ++i) {
-      ok = mbar_wait(&empty_bar[s], phase, p.status, kTimeoutEmpty);
+      ok = mbar_wait_warp(&empty_bar[s], phase, p.status, kTimeoutEmpty, &gave_up[0]);
       if (++s == kPairStages) { s = 0; phase ^= 1; }
     }
   } else if (warp == 1) {
@@ -172,12 +173,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       uint32_t phase = 0, free_phase = 1;
       bool ok = true;
       for (int t = pair; t < tiles && ok; t += pairs) {
-        ok = mbar_wait_cluster(&accum_free[buf], free_phase, p.status, kTimeoutAccum);
+        ok = mbar_wait_cluster(&accum_free[buf], free_phase, p.status, kTimeoutAccum, &gave_up[1]);
         tc_fence_after();
         const uint32_t acc = tmem_base + buf * TN;
         uint32_t more = 0;
         for (int kb = 0; kb < nkb && ok; ++kb) {
-          ok = mbar_wait_cluster(&full_bar[s], phase, p.status, kTimeoutFull);
+          ok = mbar_wait_cluster(&full_bar[s], phase, p.status, kTimeoutFull, &gave_up[1]);
           if (!ok) break;
           tc_fence_after();
           if (elect_one()) {
@@ -205,7 +206,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     int j = 0;
     for (int t = pair; t < tiles && ok; t += pairs, ++j) {
       const int buf = j & 1;
-      ok = mbar_wait(&accum_full[buf], (j >> 1) & 1, p.status, kTimeoutAccum);
+      ok = warp_ok(mbar_wait(&accum_full[buf], (j >> 1) & 1, p.status, kTimeoutAccum));
       if (!ok) break;
       tc_fence_after();
       const int n0 = (t / m_tiles) * TN;

@@ -127,6 +127,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint64_t* accum_bar = empty_bar + kStages;
   uint64_t* tmem_free = accum_bar + 1;       // grouped mode: the epilogue has drained the accumulator of a row tile
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum_bar + 2);
+  uint32_t* gave_up = tmem_slot + 2;         // of the producing and of the issuing warp; tmem_slot[1]: EPI_ALLREDUCE
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -168,6 +169,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     mbar_init(accum_bar, 1);
     mbar_init(tmem_free, 1);
+    gave_up[0] = gave_up[1] = 0;
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -245,7 +247,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const int m_tile = m_first + tj * tile_step;
       const uint32_t bytes = stage_bytes(m_tile);
       for (int i = (tj == 0 ? pre : 0); i < nkb; ++i) {
-        p_ok = mbar_wait(&empty_bar[s], phase, p.status, kTimeoutEmpty);
+        p_ok = mbar_wait_warp(&empty_bar[s], phase, p.status, kTimeoutEmpty, &gave_up[0]);
         if (!p_ok) break;
         if (elect_one()) {
           mbar_expect_tx(&full_bar[s], bytes);
@@ -265,13 +267,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     uint32_t phase = 0;
     for (int tj = 0; tj < n_tiles_cta && ok; ++tj) {
       if (tj > 0) {                 // the epilogue must have read the previous row tile out of tensor memory
-        ok = mbar_wait(tmem_free, (tj - 1) & 1, p.status, kTimeoutAccum);
+        ok = mbar_wait_warp(tmem_free, (tj - 1) & 1, p.status, kTimeoutAccum, &gave_up[1]);
         if (!ok) break;
         tc_fence_after();
       }
       uint32_t more = 0;            // 0: the accumulator starts anew
       for (int i = 0; i < nkb && ok; ++i) {
-        ok = mbar_wait(&full_bar[s], phase, p.status, kTimeoutFull);
+        ok = mbar_wait_warp(&full_bar[s], phase, p.status, kTimeoutFull, &gave_up[1]);
         if (!ok) break;
         if (lane == 0 && tj == 0 && i == 0) JS_TRACE(2);   // first stage landed
         tc_fence_after();
@@ -338,7 +340,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int grow = m0 + row;
   if (epi_warp) {
     pdl_wait();   // residual / C may be produced by the previous kernel
-    if (MT == 1 || tj == 0) acc_ok = mbar_wait(accum_bar, tj & 1, p.status, kTimeoutAccum);
+    if (MT == 1 || tj == 0) acc_ok = warp_ok(mbar_wait(accum_bar, tj & 1, p.status, kTimeoutAccum));
     tc_fence_after();
     if (threadIdx.x == 64) JS_TRACE(3);   // accumulator complete
   }
@@ -376,8 +378,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     if (threadIdx.x == 64) JS_TRACE(5);   // every peer's partial has landed here
   }
 
-  if constexpr (EPI == EPI_TOPK) {
-    // the few-rows path below synchronises the four epilogue warps with each other: all of them take it or none
+  if constexpr (EPI == EPI_TOPK || EPI == EPI_ALLREDUCE || EPI == EPI_EP_COMBINE) {
+    // the paths below synchronise the four epilogue warps with each other: all of them take them or none
     if (epi_warp) acc_ok = epi_bar_and(acc_ok);
   }
   if (epi_warp && acc_ok) {
