@@ -484,10 +484,10 @@ latent_attn_merge_kernel(const float* ws_o, const float* ws_ml, __nv_bfloat16* o
     float2 ml = make_float2(-INFINITY, 0.f);
     if (s < splits) ml = *reinterpret_cast<const float2*>(ws_ml + (static_cast<size_t>(s) * rows + row) * 2);
     const float m = warp_max(ml.x);
-    const float f = ml.x == -INFINITY ? 0.f : exp2f(ml.x - m);
+    const float f = ml.y == 0.f ? 0.f : exp2f(ml.x - (m == -INFINITY ? 0.f : m));   // NaN scores leave a sum without a maximum
     float l = warp_sum(ml.y * f);
     if (gate != nullptr) l *= 1.f + expf(-gate[static_cast<size_t>(row / H) * ldg + row % H]);
-    if (s < LMAX_SPLITS) w[s] = l > 0.f ? f / l : 0.f;
+    if (s < LMAX_SPLITS) w[s] = l > 0.f || isnan(l) ? f / l : 0.f;
   }
   __syncthreads();
   if (c >= cols) return;

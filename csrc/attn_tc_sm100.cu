@@ -864,10 +864,14 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
       float m = -INFINITY;
       for (int s2 = 0; s2 < p.splits; ++s2) m = fmaxf(m, recv_ml[(s2 * TROWS + row) * 2]);
       float wsrc[8], lsum = 0.f;
+      const float m_safe = m == -INFINITY ? 0.f : m;       // NaN scores leave a sum without a maximum
+      unsigned saw = 0;                                    // splits that saw a visible key (the others' chunks were never pushed)
       for (int s2 = 0; s2 < p.splits; ++s2) {
-        const float ms = recv_ml[(s2 * TROWS + row) * 2];
-        wsrc[s2] = (ms == -INFINITY) ? 0.f : exp2f(ms - m);
-        lsum += recv_ml[(s2 * TROWS + row) * 2 + 1] * wsrc[s2];
+        const float ls = recv_ml[(s2 * TROWS + row) * 2 + 1];
+        wsrc[s2] = exp2f(recv_ml[(s2 * TROWS + row) * 2] - m_safe);
+        if (ls == 0.f) continue;
+        saw |= 1u << s2;
+        lsum += ls * wsrc[s2];
       }
       const float inv = lsum > 0.f ? gate / lsum : 0.f;
       for (int c = split; c < 4; c += p.splits) {
@@ -875,7 +879,7 @@ __global__ void __launch_bounds__(TTHREADS, 1) paged_tree_attn_tc_kernel(AttnTcP
 #pragma unroll
         for (int j = 0; j < 32; ++j) acc[j] = 0.f;
         for (int s2 = 0; s2 < p.splits; ++s2) {
-          if (wsrc[s2] == 0.f) continue;       // that split saw no visible key (its chunk was never pushed)
+          if (!((saw >> s2) & 1u)) continue;
           const float* src = recv_o + (s2 * per_owner + c / p.splits) * 4096 + row;
 #pragma unroll
           for (int j = 0; j < 32; ++j) acc[j] += src[j * TROWS] * wsrc[s2];
@@ -918,8 +922,8 @@ __global__ void __launch_bounds__(256) diff_merge_kernel(AttnTcParams p) {
     float acc[4] = {}, l = 0.f;
     for (int s = 0; s < p.splits; ++s) {
       const float ms = p.ws_ml[(s * stride + at) * 2], ls = p.ws_ml[(s * stride + at) * 2 + 1];
-      if (ms == -INFINITY) continue;   // this split saw no visible key (its O may be unwritten)
-      const float w = exp2f(ms - top);
+      if (ls == 0.f) continue;         // this split saw no visible key (its O may be unwritten)
+      const float w = exp2f(ms - (top == -INFINITY ? 0.f : top));   // NaN scores leave a sum without a maximum
       l += ls * w;
       const float4 v = *reinterpret_cast<const float4*>(p.ws_o + (s * stride + at) * TD + lane * 4);
       acc[0] += v.x * w; acc[1] += v.y * w; acc[2] += v.z * w; acc[3] += v.w * w;

@@ -406,6 +406,31 @@ def test_paged_attention_of_two_softmax_groups(ext, Hq, Hkv, splits, causal):
     ext.check_status("cuda")
 
 
+@pytest.mark.parametrize("splits", [1, 2, 3, 4, 8, 12])
+@pytest.mark.parametrize("maps", [1, 2])
+def test_rows_of_nan_scores_stay_nan(ext, splits, maps):
+    """A row whose scores are all NaN has a sum and no maximum: however many key splits, merged in a cluster or by a launch of its
+    own, its output is NaN and every other row's is what it was."""
+    H, G, past, n = 8, 2, 900, 5
+    q, kp, vp = rnd(n, H, 128, seed=90), rnd(G, 1024, 128, seed=91), rnd(G, 1024, 128, seed=92)
+    smap = torch.randperm(1024, device="cuda").to(torch.int32).view(1, -1)
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    args = (smap, i32(0), i32(0, n), i32(past), None, 0.15, 0, False, True)
+    ws = {"o": torch.full((splits, n, maps * H, 128), 7.0, device="cuda"), "ml": torch.full((splits, n, maps * H, 2), 7.0, device="cuda")}
+    kw = dict(diff=(torch.tensor([0.55], device="cuda"), 0.65, 1e-4), vdim=128) if maps == 2 else {}
+    outs = []
+    for bad in (False, True):
+        if bad:
+            q[2, 3] = float("nan")
+        out = torch.zeros(n, H * 128, dtype=torch.bfloat16, device="cuda")
+        ext.window_attention_tc(q, kp, vp, *args, out, splits=splits, ws=ws, **kw)
+        outs.append(out.view(n, H, 128))
+    hit = torch.zeros(n, H, dtype=torch.bool, device="cuda")
+    hit[2, 3] = True
+    assert torch.isnan(outs[1][hit]).all() and torch.equal(outs[1][~hit], outs[0][~hit]) and torch.isfinite(outs[0]).all()
+    ext.check_status("cuda")
+
+
 @pytest.mark.parametrize("seed", range(4))
 def test_device_tree_build_and_accept_match_host(ext, seed):
     import ctypes

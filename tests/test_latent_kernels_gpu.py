@@ -162,6 +162,18 @@ def test_latent_attention_tensor_cores(ext, H, R, counts, pasts, splits, tree):
     close(out, c["want"])
 
 
+@pytest.mark.parametrize("splits", [1, 3])
+def test_latent_rows_of_nan_scores_stay_nan(ext, splits):
+    c = latent_case(16, 320, [3, 1], [127, 500], False)
+    c["q"][5] = float("nan")
+    out = ext.latent_attention_rows(c["q"], c["pool"], 16, c["slot_map"], c["rows"], c["cu"], c["past"], None, c["scale"], True, c["max_q"],
+                                    splits=splits, impl="tc")
+    ext.check_status(DEV)
+    rest = torch.arange(len(out), device=DEV) != 5
+    assert torch.isnan(out[5]).all()
+    close(out[rest], c["want"][rest])
+
+
 @pytest.mark.parametrize("H,R,counts,pasts", CASES + [(2, 700, [5, 1], [40, 9])])
 @pytest.mark.parametrize("dtype,tol", [(torch.float32, 2e-6), (torch.bfloat16, 8e-3)])
 @pytest.mark.parametrize("tree", [False, True])
