@@ -342,7 +342,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     pdl_wait();   // residual / C may be produced by the previous kernel
     if (MT == 1 || tj == 0) acc_ok = warp_ok(mbar_wait(accum_bar, tj & 1, p.status, kTimeoutAccum));
     tc_fence_after();
-    if (threadIdx.x == 64) JS_TRACE(3);   // accumulator complete
+    if (row == 0) JS_TRACE(3);   // accumulator complete (the warp of the first 32 rows takes part in every form)
   }
 
   if (split > 1) {

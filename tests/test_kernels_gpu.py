@@ -215,6 +215,16 @@ def test_gemm_split_pushes_meet_started_peers(ext, M, deep, split):
     ext.check_status("cuda")
 
 
+@pytest.mark.parametrize("M,split", [(1, 1), (16, 4), (17, 2), (100, 1), (128, 4)])
+def test_gemm_phase_timestamps(ext, M, split):
+    """All phases of the first CTA leave a time stamp, also where only the warps of the valid rows have an epilogue."""
+    x, w = rnd(M, 1024, seed=84), rnd(256, 1024, scale=0.05, seed=85)
+    trace = torch.zeros(8, dtype=torch.int64, device="cuda")
+    ext.gemm(x, w, bn=128, split=split, deep=1, trace=trace)
+    stamps = [t for i, t in enumerate(trace.tolist()) if split > 1 or i not in (4, 5)]
+    assert min(stamps) > 0 and stamps[0] == min(stamps) and stamps[-1] == max(stamps)
+
+
 def test_gemm_fp32_out(ext):
     x, w = rnd(64, 512, seed=6), rnd(128, 512, scale=0.05, seed=7)
     out = ext.gemm(x, w, epi=ext.EPI_STORE_F32, split=2)
