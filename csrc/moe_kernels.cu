@@ -232,8 +232,9 @@ extern "C" int js_moe_sort_inv(const int* idx, const float* wts, int P, int E, i
   if (P <= 0) return 0;
   if (k < 1) return -10;
   if (P > js::kSortMaxPairs || n_local < 1 || E < 1) return -10;
-  // as many slices as 160 KB of counts allow (all 32 up to 1279 local experts)
-  const int slices = (40 * 1024) / (n_local + 1) < 1 ? 1 : (40 * 1024) / (n_local + 1) > js::kSortThreads / 32 ? js::kSortThreads / 32 : (40 * 1024) / (n_local + 1);
+  // as many slices as shared memory has room for counts (all 32 up to 1708 experts, all local)
+  const int fit = (227 * 256 - (n_local + 2) - E) / (n_local + 1);
+  const int slices = fit < 1 ? 1 : fit > js::kSortThreads / 32 ? js::kSortThreads / 32 : fit;
   const int smem = (slices * (n_local + 1) + n_local + 2 + E) * 4;
   static int configured[js::kMaxDevicesCached] = {};
   if (js::ensure_dyn_smem(js::moe_sort_kernel, smem, configured) != 0) return -3;

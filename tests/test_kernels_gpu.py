@@ -441,6 +441,23 @@ def test_rows_of_nan_scores_stay_nan(ext, splits, maps):
     ext.check_status("cuda")
 
 
+@pytest.mark.parametrize("E,P", [(1, 40), (128, 16384), (1708, 500), (1709, 500), (13000, 64), (19000, 64)])
+def test_pair_sort_takes_what_fits_in_shared_memory(ext, E, P):
+    """From all slices down to one: sorted stably by expert, with the experts' offsets and counts."""
+    import ctypes
+    idx = torch.randint(0, E, (P,), generator=torch.Generator().manual_seed(E)).to(torch.int32)
+    wts = torch.rand(P)
+    new = lambda n, t=torch.int32: torch.empty(n, dtype=t, device="cuda")
+    order, row_w, off, cnt, d_idx, d_wts = new(P), new(P, torch.float32), new(E + 1), new(E), idx.cuda(), wts.cuda()
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    ext._check(ext.load().js_moe_sort(p(d_idx), p(d_wts), P, E, 0, E, p(order), p(row_w), p(off), p(cnt), 1, None, 0, ext._stream()), "js_moe_sort")
+    want = torch.argsort(idx, stable=True)
+    assert torch.equal(order.cpu(), want.to(torch.int32)) and torch.equal(row_w.cpu(), wts[want])
+    counts = torch.bincount(idx, minlength=E)
+    assert torch.equal(cnt.cpu(), counts.to(torch.int32))
+    assert off[0] == 0 and torch.equal(off.cpu()[1:], counts.cumsum(0).to(torch.int32))
+
+
 @pytest.mark.parametrize("seed", range(4))
 def test_device_tree_build_and_accept_match_host(ext, seed):
     import ctypes
