@@ -972,6 +972,7 @@ static int launch_attn_tc(const AttnTcParams& p, const AttnMaps& maps, int q_til
 
 // Tensor maps of the pools, or false for a layout that no such map describes.
 static bool make_attn_maps(AttnMaps* m, const void* k, const void* v, int Hkv, int S, long long kv_head, long long kv_slot) {
+  if (kv_slot < TD) return false;                                // overlapping or repeated slots
   uint64_t rows = S, cols = TD;
   m->head_rows = m->head_cols = 0;
   if (Hkv > 1) {
@@ -985,7 +986,7 @@ static bool make_attn_maps(AttnMaps* m, const void* k, const void* v, int Hkv, i
       return false;
     }
   }
-  return kv_slot >= TD && rows < (1ull << 31) && !make_map(&m->k16, k, rows, cols, kv_slot, 16) && !make_map(&m->v16, v, rows, cols, kv_slot, 16) &&
+  return rows < (1ull << 31) && !make_map(&m->k16, k, rows, cols, kv_slot, 16) && !make_map(&m->v16, v, rows, cols, kv_slot, 16) &&
          !make_map(&m->k1, k, rows, cols, kv_slot, 1) && !make_map(&m->v1, v, rows, cols, kv_slot, 1);
 }
 

@@ -416,6 +416,30 @@ def test_paged_attention_of_two_softmax_groups(ext, Hq, Hkv, splits, causal):
     ext.check_status("cuda")
 
 
+@pytest.mark.parametrize("layout", ["one row for all keys", "wider rows", "overlapping rows"])
+def test_attention_over_rows_of_any_stride(ext, layout):
+    """Key and value matrices that no tensor map describes take the other loaders: a single row seen as many (stride 0), rows that
+    overlap; and a column block of a wider matrix, which has a map."""
+    from jetspec_b200.ops import reference as ref
+    G, H, past, n = 2, 8, 200, 7
+    L = past + n
+    if layout == "one row for all keys":
+        k, v = (rnd(1, G * 128, seed=s).expand(L, G * 128) for s in (95, 96))
+    elif layout == "wider rows":
+        k, v = (rnd(L, G * 128 + 64, seed=s)[:, :G * 128] for s in (95, 96))
+    else:
+        k, v = (torch.as_strided(rnd(L * 64 + 512, 1, seed=s).view(-1), (L, G * 128), (64, 1)) for s in (95, 96))
+    q = rnd(n, H, 128, seed=97)
+    smap = torch.randperm(L, device="cuda").to(torch.int32).view(1, -1)
+    i32 = lambda *x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    out = torch.empty(n, H * 128, dtype=torch.bfloat16, device="cuda")
+    ext.paged_attention_rows(q, k, v, smap, i32(0), i32(0, n), i32(past), 0.1, n, out, L)
+    pool = lambda t: t.reshape(L, G, 128).transpose(0, 1).float().contiguous()
+    want = ref.paged_tree_attention(q.float(), pool(k), pool(v), smap, i32(0), i32(0, n), i32(past), None, 0.1, True)
+    assert rel_err(out, want) < BF16_TOL
+    ext.check_status("cuda")
+
+
 @pytest.mark.parametrize("splits", [1, 2, 3, 4, 8, 12])
 @pytest.mark.parametrize("maps", [1, 2])
 def test_rows_of_nan_scores_stay_nan(ext, splits, maps):
