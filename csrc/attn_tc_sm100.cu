@@ -1076,7 +1076,8 @@ extern "C" int js_window_attention_tc(const void* q, const void* k_pool, const v
       if (dev >= 0 && dev < kMaxDevicesCached) room[dev][gi][splits] = r;
     }
     const int npt = 128 / G;
-    in_cluster = r > 0 && ((T + npt - 1) / npt) * Hkv <= r;
+    const int tiles = (T + npt - 1) / npt;
+    in_cluster = r > 0 && (tiles > B ? tiles : B) * Hkv <= r;      // a tile's rows are one sequence's
   }
   // Two softmax groups where a CTA has many tiles: without splits (many query rows), or with long ones.  A decode round's
   // splits hold a few tiles each, and merging in the cluster counts for more there.

@@ -128,7 +128,7 @@ class _Stack:
         self.attn = torch.zeros(T, Hq * D, **bf)
         self.act = torch.zeros(T, I, **bf)
         self._q4: dict = {}
-        self.splits = X.attn_splits_for(T, Hq, Hkv, max_keys, seqs)
+        self.seqs, self.splits = seqs, X.batch_attn_splits(T, Hq, Hkv, max_keys, seqs)
         self.attn_ws = None
         if self.splits > 1:
             self.attn_ws = {"o": torch.zeros(self.splits, T, Hq, D, dtype=torch.float32, device=device),
@@ -206,7 +206,7 @@ def decoder_layers(cfg, layers, st: _Stack, k_pools, v_pools, slot_map, seq_rows
     n = 0
     # the split merge is a second launch unless the tcgen05 kernel does it inside a cluster
     in_kernel = (X.attn_impl(Hq, Hkv, 0 if mask_bits is None else mask_bits.shape[1]) == "tc"
-                 and X.attn_merges_in_cluster(st.T, Hq, Hkv, st.splits))
+                 and X.attn_merges_in_cluster(st.T, Hq, Hkv, st.splits, st.seqs))
     merge_launch = 1 if st.splits > 1 and not in_kernel else 0
     fuse_norm = tp is not None and tp.push_only >= 2     # the all-reduce tail computes the following norm
     h_ready = False                                      # st.h already holds this layer's normalised input

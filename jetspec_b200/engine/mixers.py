@@ -120,7 +120,8 @@ class WindowMixer:
             splits = X.window_attn_splits(T, Hq, c.kv_heads, batch.max_keys, c.window, c.keep_first, c.pool, batch.seq_rows.numel())
             X.window_attention_tc(q.view(T, Hq, 128), kp, vp, *args, c.scale, c.window, self.sink, batch.mask is None, o, splits=splits,
                                   ws=split_ws(st, splits, T * Hq * c.maps, 128), pdl=pdl, **more)
-            n += int(splits > 1 and (self.diff is not None or not X.attn_merges_in_cluster(T, Hq, c.kv_heads, splits)))
+            n += int(splits > 1 and (self.diff is not None or not X.attn_merges_in_cluster(T, Hq, c.kv_heads, splits,
+                                                                                                   batch.seq_rows.numel())))
         else:
             X.window_attention(q.view(T, Hq * c.maps, self.Dq), kp, vp, self.vq, *args, c.scale, c.window, self.sink, batch.mask is None, out=o,
                                pdl=pdl, norm_dim=c.vdim, **more)

@@ -21,6 +21,7 @@ from __future__ import annotations
 
 import ctypes
 import glob
+import math
 import os
 import subprocess
 import sys
@@ -591,7 +592,7 @@ def _attn_cluster_room(G: int, splits: int) -> int:
     return _ATTN_ROOM[key]
 
 
-def attn_merges_in_cluster(T: int, Hq: int, Hkv: int, splits: int) -> bool:
+def attn_merges_in_cluster(T: int, Hq: int, Hkv: int, splits: int, seqs: int = 1) -> bool:
     """Whether the tcgen05 kernel merges ``splits`` key splits itself (they form one cluster and exchange partial
     outputs through distributed shared memory): up to ATTN_CLUSTER_SPLITS, and only while all clusters of the
     launch are resident at once (a cluster lives inside one GPC: 148 SMs hold 33 clusters of 4 but only 15 of 8)."""
@@ -599,7 +600,7 @@ def attn_merges_in_cluster(T: int, Hq: int, Hkv: int, splits: int) -> bool:
     if attn_impl(Hq, Hkv) != "tc" or not 2 <= splits <= ATTN_CLUSTER_SPLITS:
         return False
     npt = 128 // G
-    return ((T + npt - 1) // npt) * Hkv <= _attn_cluster_room(G, splits)
+    return max((T + npt - 1) // npt, seqs) * Hkv <= _attn_cluster_room(G, splits)      # a tile's rows are one sequence's
 
 
 def attn_splits_for(T: int, Hq: int, Hkv: int, max_keys: int, seqs: int = 1) -> int:
@@ -615,6 +616,22 @@ def attn_splits_for(T: int, Hq: int, Hkv: int, max_keys: int, seqs: int = 1) -> 
         return max(1, min(SM_COUNT // ctas, (max_keys + 127) // 128, 16))
     npt = max(1, 64 // G)
     return attn_splits((T + npt - 1) // npt, Hkv, max_keys)
+
+
+def batch_attn_splits(T: int, Hq: int, Hkv: int, max_keys: int, seqs: int) -> int:
+    """Key splits for a batch of ``seqs`` sequences of unknown lengths up to ``max_keys``.
+
+    Where rows fill tiles of their own accord this is :func:`attn_splits_for`.  More sequences than that mean as many
+    tiles, each with few rows.  Their splits then run in several waves, most of them empty where lengths differ, while the longest
+    sequence is one chain of key tiles: about ``0.77 (max_keys / 64) / splits + 4 (seqs * Hkv * splits / 148)`` microseconds,
+    which is least at the root below.  Rows of one token, 32 query and 8 KV heads (microseconds; one wave's splits as for a
+    single sequence / one wave's splits over all sequences / this rule): one of 12000 keys and nine of 300 67 / 163 / 58,
+    12 of 100 - 3000 79 / 40 / 50, 18 of 2000 138 / 46 / 56, one of 12000 and 39 of 300 128 / 177 / 118, one of 4000 and 31 of 500
+    134 / 79 / 75, one of 12000 and two of 300 48 / 46 / 47."""
+    most = attn_splits_for(T, Hq, Hkv, max_keys)
+    if attn_impl(Hq, Hkv) != "tc" or seqs <= (T * (Hq // Hkv) + 127) // 128:
+        return most
+    return max(1, min(most, math.isqrt(int(0.44 * max_keys / (seqs * Hkv)))))
 
 
 def paged_tree_attention(q, k_pool, v_pool, slot_map, seq_rows, cu_q, past_lens, mask_bits, scale: float,
@@ -633,7 +650,7 @@ def paged_tree_attention(q, k_pool, v_pool, slot_map, seq_rows, cu_q, past_lens,
         out = torch.empty(T, Hq * D, dtype=q.dtype, device=q.device)
     if splits is None:
         mk = max_keys if max_keys is not None else slot_map.shape[1]
-        splits = attn_splits_for(T, Hq, Hkv, mk, B)
+        splits = batch_attn_splits(T, Hq, Hkv, mk, B)
     ws_o = ws_ml = None
     if splits > 1:
         if ws is None:

@@ -101,6 +101,15 @@ def test_kernel_config_pickers_on_cpu():
     assert X.attn_splits_for(128, 32, 8, 2700) == 4
     assert X.attn_splits_for(128, 4, 1, 2700) == 16
     assert X.attn_splits_for(2048, 32, 8, 2700) == 1
+    # batches of more sequences than row tiles: the longest may hold nearly all keys, so more splits the longer it can be,
+    # fewer the more sequences there are, and never more than for one sequence
+    assert X.batch_attn_splits(10, 32, 8, 12288, 10) == 8 and X.batch_attn_splits(40, 32, 8, 12288, 40) == 4
+    assert X.batch_attn_splits(24, 32, 8, 512, 24) == 1 and X.batch_attn_splits(12, 16, 1, 12288, 12) == 16
+    assert X.batch_attn_splits(128, 32, 8, 2700, 4) == 4 and X.batch_attn_splits(512, 32, 8, 12288, 4) == 1
+    for T, seqs, keys in ((1, 1, 64), (10, 10, 12288), (24, 24, 4096), (100, 5, 12288), (64, 64, 1024), (7, 7, 100)):
+        for Hq, Hkv in ((32, 8), (8, 8), (16, 1)):
+            assert 1 <= X.batch_attn_splits(T, Hq, Hkv, keys, seqs) <= X.attn_splits_for(T, Hq, Hkv, keys)
+    assert X.attn_merges_in_cluster(10, 32, 8, 4) and not X.attn_merges_in_cluster(10, 32, 8, 4, 10)
     # in-cluster merge: up to 8 splits and only while every cluster of the launch is resident at once
     assert X.attn_merges_in_cluster(128, 32, 8, 4)
     assert not X.attn_merges_in_cluster(128, 32, 8, 16)

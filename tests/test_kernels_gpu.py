@@ -416,6 +416,24 @@ def test_paged_attention_of_two_softmax_groups(ext, Hq, Hkv, splits, causal):
     ext.check_status("cuda")
 
 
+@pytest.mark.parametrize("lens", [[2900] + [30] * 9, [700, 3, 650], [1] * 40, list(range(1, 400, 17))])
+def test_batch_of_unequal_lengths(ext, lens):
+    """One new token of each of many sequences, key splits as picked for the batch: splits without a key tile, merged by a launch."""
+    from jetspec_b200.ops import reference as ref
+    B, Hq, Hkv = len(lens), 32, 8
+    S, width = sum(lens) + B, (max(lens) + 128) // 64 * 64
+    q, kp, vp = rnd(B, Hq, 128, seed=98), rnd(Hkv, S, 128, seed=99), rnd(Hkv, S, 128, seed=100)
+    smap, perm, off = torch.zeros(B, width, dtype=torch.int32, device="cuda"), torch.randperm(S, device="cuda").to(torch.int32), 0
+    for b, n in enumerate(lens):
+        smap[b, :n + 1] = perm[off:off + n + 1]
+        off += n + 1
+    cu, rows = torch.arange(B + 1, dtype=torch.int32, device="cuda"), torch.arange(B, dtype=torch.int32, device="cuda")
+    past = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    out = ext.paged_tree_attention(q, kp, vp, smap, rows, cu, past, None, 0.1, True, 1)
+    assert rel_err(out, ref.paged_tree_attention(q.float(), kp.float(), vp.float(), smap, rows, cu, past, None, 0.1, True)) < BF16_TOL
+    ext.check_status("cuda")
+
+
 @pytest.mark.parametrize("layout", ["one row for all keys", "wider rows", "overlapping rows"])
 def test_attention_over_rows_of_any_stride(ext, layout):
     """Key and value matrices that no tensor map describes take the other loaders: a single row seen as many (stride 0), rows that
