@@ -108,6 +108,23 @@ def _finish_layer_weights(out: list) -> list:
     return out
 
 
+_WIDE_GU_ROWS = 1024
+
+
+def _gu_weight(L: dict, rows: int, tp) -> tuple:
+    """``(weight, its interleave)`` of the layer's gate/up product for ``rows`` rows.  Weights in 192-row blocks
+    (``JETSPEC_GU_TILE=192``) suit one wave of 192-column tiles of a decode round; CTA pairs have no such tile, and 2048 rows of
+    Qwen3-8B's take 388 us and more on single CTAs against 269 on pairs.  A second copy in blocks of 256 is made on
+    first use from 1024 rows on."""
+    if rows < _WIDE_GU_ROWS or tp is not None or L.get("gu_bn") != 192 or L["gu"].shape[0] % 256:
+        return L["gu"], L.get("gu_bn")
+    if "gu256" not in L:
+        I2, H = L["gu"].shape
+        v = L["gu"].view(I2 // 192, 2, 96, H)
+        L["gu256"] = X.interleave_gate_up(v[:, 0].reshape(I2 // 2, H), v[:, 1].reshape(I2 // 2, H), 256)
+    return L["gu256"], 256
+
+
 # Rows of a prefill portion: wide enough that its GEMMs are bound by the tensor cores (a layer of Qwen3-8B's: 537 us for one
 # portion of 2048 rows, 4 x 171 for four of 512), few enough that the activations stay in the tens of megabytes.
 _PREFILL_ROWS = 2048
@@ -271,7 +288,8 @@ def decoder_layers(cfg, layers, st: _Stack, k_pools, v_pools, slot_map, seq_rows
             continue
         if pf is not None:
             pf.ahead(L["down"])
-        X.gemm(st.h, L["gu"], out=st.act, epi=X.EPI_SWIGLU, bn=L.get("gu_bn"), pdl=pdl)
+        gu, bn = _gu_weight(L, st.T, tp)
+        X.gemm(st.h, gu, out=st.act, epi=X.EPI_SWIGLU, bn=bn, pdl=pdl)
         if pf is not None:
             nxt = layers[li + 1]["qkv"] if li != last else then_prefetch
             if nxt is not None:

@@ -86,6 +86,24 @@ def test_llm_round_collector_runs_on_the_reference_engine_path():
             assert out["verdict"] in ("P3_BUILD", "P3_SKIP") and "lift" in out
 
 
+def test_gate_up_in_192_row_blocks_goes_wide_for_many_rows():
+    """JETSPEC_GU_TILE=192: from 1024 rows on the product runs on a copy in blocks of 256, which CTA pairs take."""
+    import torch
+    from jetspec_b200.engine.fast_round import _gu_weight
+    from jetspec_b200.ops import cuda_ext as X
+    g, u = torch.randn(768, 16), torch.randn(768, 16)
+    L = {"gu": X.interleave_gate_up(g, u, 192), "gu_bn": 192}
+    assert _gu_weight(L, 1023, None) == (L["gu"], 192) and _gu_weight(L, 2048, object()) == (L["gu"], 192)
+    w, bn = _gu_weight(L, 1024, None)
+    assert bn == 256 and torch.equal(w, X.interleave_gate_up(g, u, 256)) and _gu_weight(L, 4096, None)[0] is w
+    assert X.pick_pair_tile(2048, 24576, 4096, 192) == 0 and X.pick_pair_tile(2048, 24576, 4096, bn) == 256
+    for bn in (128, 256, None):
+        M = {"gu": L["gu"], "gu_bn": bn}
+        assert _gu_weight(M, 4096, None) == (L["gu"], bn)
+    odd = {"gu": X.interleave_gate_up(g[:96], u[:96], 192), "gu_bn": 192}
+    assert _gu_weight(odd, 4096, None)[1] == 192
+
+
 def test_kernel_config_pickers_on_cpu():
     """Host-side launch policies that need no GPU: the GEMM picker's many-row rule and the attention split count."""
     from jetspec_b200.ops import cuda_ext as X
