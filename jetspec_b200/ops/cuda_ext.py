@@ -232,8 +232,18 @@ def gu_tile(intermediate: int) -> int:
     return int(env) if env else 128
 
 
+def _k_split(tiles: int, kb: int) -> int:
+    """CTAs of a cluster that share the K range of one of ``tiles`` tiles, ``kb`` 64-wide k-blocks deep.
+
+    Measured on chains of L2-cold GEMMs (M = 128): a K split helps while the whole grid is one wave of one CTA per SM AND the
+    clusters can be placed (a cluster lives inside one GPC, so only ~32 clusters of 4, ~40 of 3 or ~72 of 2 fit at
+    once; 48 clusters of 3 ran as two waves)."""
+    room = {2: 72, 3: 40, 4: 32}
+    return next((c for c in (4, 3, 2) if tiles <= room[c] and tiles * c <= SM_COUNT and kb // c >= 4), 1)
+
+
 def pick_gemm_config(M: int, N: int, K: int, epi: int, bn: Optional[int] = None):
-    """``(bn, split, deep)``: tile width, K-split cluster size, pipeline variant.
+    """``(bn, split, deep)`` of a launch on single CTAs: tile width, K-split cluster size, pipeline variant.
 
     Decode shapes are weight-streaming bound, so the goal is enough CTAs to cover the
     SMs (two CTAs fit per SM with the shallow pipeline) without re-reading the
@@ -243,18 +253,6 @@ def pick_gemm_config(M: int, N: int, K: int, epi: int, bn: Optional[int] = None)
     if key in GEMM_TUNING:
         return GEMM_TUNING[key]
     m_tiles = (M + 127) // 128
-    if bn is None and epi == EPI_STORE and m_tiles >= 4 and N % 256 == 0 and m_tiles * (N // 256) >= 64:
-        # prefill / batched verify (>= 512 rows): compute bound, and a 128x128 tile asks more of the L2-to-SM path
-        # than it gives; 128x256 tiles with the deep pipeline measured 5-12 % faster at 2048 rows
-        # (qkv 97 -> 91 us, o 62 -> 56, down 182 -> 165) and equal or better at 512.  From 1024 rows on, two row tiles
-        # per CTA (deep = 3: 256 x 256 outputs per CTA, every weight stage feeds two accumulators) when that does not
-        # cost a wave: at 2048 rows o 53.9 -> 48.7 us, down 155.4 -> 146.3 (128 CTAs, one wave), but qkv
-        # 88.1 -> 96.2 (192 CTAs: two waves of big tiles against three of small ones), gate/up equal.
-        if m_tiles >= 8:
-            t1, t2 = m_tiles * (N // 256), ((m_tiles + 1) // 2) * (N // 256)
-            if 2 * ((t2 + SM_COUNT - 1) // SM_COUNT) <= (t1 + SM_COUNT - 1) // SM_COUNT:
-                return 256, 1, 3
-        return 256, 1, 1
     bn = bn or 128
     tiles = m_tiles * ((N + bn - 1) // bn)
     kb = (K + 63) // 64
@@ -262,15 +260,7 @@ def pick_gemm_config(M: int, N: int, K: int, epi: int, bn: Optional[int] = None)
     if epi in (EPI_STORE, EPI_STORE_F32, EPI_SWIGLU):
         # SwiGLU tiles hold two (gate, up) chunk pairs, so a split of 4 leaves two CTAs of each cluster without
         # output columns; it still pays when the projection is narrow (tensor-parallel shards: 24 tiles -> 96 CTAs)
-        max_split = 4
-        # Measured on chains of L2-cold GEMMs (M = 128): a K split helps while the whole grid is one
-        # wave of one CTA per SM AND the clusters can be placed (a cluster lives inside one GPC, so only
-        # ~32 clusters of 4, ~40 of 3 or ~72 of 2 fit at once; 48 clusters of 3 ran as two waves).
-        room = {2: 72, 3: 40, 4: 32}
-        for c in (4, 3, 2):
-            if c <= max_split and tiles <= room[c] and tiles * c <= SM_COUNT and kb // c >= 4:
-                split = c
-                break
+        split = _k_split(tiles, kb)
     if split > 1:
         # deep pipeline (192 KB, one CTA per SM; the receive area aliases the stages), except for the narrow shards of
         # a tensor-parallel rank (at most 96 CTAs with at most 16 k-blocks each): 128 KB serves those as well and
@@ -296,13 +286,14 @@ def pick_pair_tile(M: int, N: int, K: int, interleave: int = 128) -> int:
     columns (the tensor pipe) and 0.19 on 128 columns (the L2-to-SM path); single CTAs 0.235 on 128 x 128 tiles, which can
     split K.  At 2048 rows (microseconds, single CTAs against pairs): 4096 x 6144 91.6 / 78.8, 4096 x 24576 388 / 269,
     4096 x 151936 2037 / 1542; at 512 rows 4096 x 24576 124 / 79, 12288 x 4096 70 / 47; but at 256 rows 12288 x 4096 with
-    K split in two 30.6 / 42."""
+    K split in two 30.6 / 42.  Where single CTAs are taken their tiles are 128 columns wide, as weighed here: 4096 x 3328
+    at 640 rows 27.6, 35.8 on 256 columns; 4096 x 2048 at 1152 rows 27.6 / 33.8."""
     if M <= 128 or interleave not in (128, 256):
         return 0
     rows, single = (M + 255) // 256, (M + 127) // 128 * ((N + 127) // 128)
     passes = lambda tiles: (tiles + SM_PAIRS - 1) // SM_PAIRS
     wide, narrow = 0.285 * passes(rows * ((N + 255) // 256)), 0.19 * passes(rows * ((N + 127) // 128))
-    if single <= SM_COUNT and 0.235 / pick_gemm_config(128, single * 128, K, EPI_STORE, 128)[1] <= min(wide, narrow):
+    if single <= SM_COUNT and 0.235 / _k_split(single, (K + 63) // 64) <= min(wide, narrow):
         return 0
     return 128 if narrow < wide and interleave == 128 else 256
 

@@ -110,11 +110,15 @@ def test_kernel_config_pickers_on_cpu():
     # decode: one row tile, weight streaming -> K split over a cluster while the grid stays one wave
     assert X.pick_gemm_config(128, 4096, 4096, X.EPI_STORE)[:2] == (128, 4)
     assert X.pick_gemm_config(128, 6144, 4096, X.EPI_STORE)[:2] == (128, 2)
-    # many rows: 256-column tiles; two row tiles per CTA only where that does not add a wave of (bigger) tiles
-    assert X.pick_gemm_config(2048, 4096, 4096, X.EPI_STORE) == (256, 1, 3)
-    assert X.pick_gemm_config(2048, 4096, 12288, X.EPI_STORE) == (256, 1, 3)
-    assert X.pick_gemm_config(2048, 6144, 4096, X.EPI_STORE) == (256, 1, 1)
-    assert X.pick_gemm_config(512, 4096, 4096, X.EPI_STORE) == (256, 1, 1)
+    # more than 128 rows: CTA pairs on 256 columns, on 128 where half as wide tiles save a pass
+    assert X.pick_pair_tile(128, 24576, 4096) == 0 and X.pick_pair_tile(129, 24576, 4096) == 256
+    assert X.pick_pair_tile(2048, 6144, 4096) == 256 and X.pick_pair_tile(512, 4096, 4096) == 128
+    assert X.pick_pair_tile(512, 24576, 4096, 256) == 256 and X.pick_pair_tile(2000, 1024, 512, 256) == 256
+    assert X.pick_pair_tile(2048, 24576, 4096, 64) == X.pick_pair_tile(2048, 24576, 4096, 192) == 0
+    # ... and single CTAs where those can split K, or fill the SMs with one tile each: 128 columns, what the rule weighs
+    assert X.pick_pair_tile(256, 4096, 12288) == 0 and X.pick_gemm_config(256, 4096, 12288, X.EPI_STORE)[:2] == (128, 2)
+    for M, N in ((640, 3328), (640, 3584), (896, 2560), (1152, 2048), (4736, 512)):
+        assert X.pick_pair_tile(M, N, 4096) == 0 and X.pick_gemm_config(M, N, 4096, X.EPI_STORE) == (128, 1, 1)
     # attention: one wave of CTAs; 32 query tiles x heads leave 4 key splits, a shard with one KV head gets 16
     assert X.attn_splits_for(128, 32, 8, 2700) == 4
     assert X.attn_splits_for(128, 4, 1, 2700) == 16
