@@ -278,9 +278,10 @@ def pick_gemm_config(M: int, N: int, K: int, epi: int, bn: Optional[int] = None)
 SM_PAIRS = SM_COUNT // 2
 
 
-def pick_pair_tile(M: int, N: int, K: int, interleave: int = 128) -> int:
-    """Width of the 256-row tiles of the CTA-pair GEMM, or 0 where single CTAs are as fast: the least number of k-blocks
-    that pass one after the other, weighed with what a 64-wide k-block takes.
+def pick_pair_tile(M: int, N: int, K: int, interleave: int = 128, epi: int = EPI_STORE) -> int:
+    """Width of the 256-row tiles of the CTA-pair GEMM, or 0 where single CTAs are as fast (or :data:`GEMM_TUNING` names a
+    configuration of theirs): the least number of k-blocks that pass one after the other, weighed with what a
+    64-wide k-block takes.
 
     Measured slopes (microseconds a k-block, 4096 x 4096 and 4096 x 12288 weights at 256 and 512 rows): pairs 0.285 on 256
     columns (the tensor pipe) and 0.19 on 128 columns (the L2-to-SM path); single CTAs 0.235 on 128 x 128 tiles, which can
@@ -288,7 +289,7 @@ def pick_pair_tile(M: int, N: int, K: int, interleave: int = 128) -> int:
     4096 x 151936 2037 / 1542; at 512 rows 4096 x 24576 124 / 79, 12288 x 4096 70 / 47; but at 256 rows 12288 x 4096 with
     K split in two 30.6 / 42.  Where single CTAs are taken their tiles are 128 columns wide, as weighed here: 4096 x 3328
     at 640 rows 27.6, 35.8 on 256 columns; 4096 x 2048 at 1152 rows 27.6 / 33.8."""
-    if M <= 128 or interleave not in (128, 256):
+    if M <= 128 or interleave not in (128, 256) or (M, N, K, epi) in GEMM_TUNING:
         return 0
     rows, single = (M + 255) // 256, (M + 127) // 128 * ((N + 127) // 128)
     passes = lambda tiles: (tiles + SM_PAIRS - 1) // SM_PAIRS
@@ -312,7 +313,7 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None,
     assert w.shape[1] == K and x.stride(1) == 1 and w.stride(1) == 1
     if pair is None:
         free = split is None and deep is None and trace is None and (bn is None or epi == EPI_SWIGLU)
-        pair = pick_pair_tile(M, N, K, bn or 128) if free and epi in (EPI_STORE, EPI_SWIGLU) and N % 8 == 0 else 0
+        pair = pick_pair_tile(M, N, K, bn or 128, epi) if free and epi in (EPI_STORE, EPI_SWIGLU) and N % 8 == 0 else 0
     if not pair:
         cb, cs, cd = pick_gemm_config(M, N, K, epi, bn)
         bn = bn or cb
@@ -435,7 +436,7 @@ def lm_head_argmax(h: torch.Tensor, w: torch.Tensor, ws: Optional[dict] = None, 
         ws = {"val": torch.empty(M, nt, dtype=torch.float32, device=h.device),
               "idx": torch.empty(M, nt, dtype=torch.int32, device=h.device)}
     gemm(h, w, out=None, epi=EPI_ARGMAX, bn=128, split=1, pdl=pdl, part_val=ws["val"], part_idx=ws["idx"],
-         pair=pick_pair_tile(M, N, h.shape[1]))
+         pair=pick_pair_tile(M, N, h.shape[1], 128, EPI_ARGMAX))
     if out_idx is None:
         out_idx = torch.empty(M, dtype=torch.int32, device=h.device)
     if out_val is None:
@@ -913,7 +914,7 @@ def gemm_inproj(x, w, raw: Optional[torch.Tensor], n_raw: int, act_out: Optional
     M, K = x.shape
     N = w.shape[0]
     if bn is None:
-        tn = pick_pair_tile(M, N, K)
+        tn = pick_pair_tile(M, N, K, 128, EPI_SWIGLU)
         if tn:
             _check(lib.js_gemm_inproj_pair(_p(x), _p(w), _p(raw), _p(act_out), M, N, K, x.stride(0), w.stride(0),
                                            raw.stride(0) if raw is not None else 0, act_out.stride(0) if act_out is not None else 0,

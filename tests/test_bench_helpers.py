@@ -119,6 +119,13 @@ def test_kernel_config_pickers_on_cpu():
     assert X.pick_pair_tile(256, 4096, 12288) == 0 and X.pick_gemm_config(256, 4096, 12288, X.EPI_STORE)[:2] == (128, 2)
     for M, N in ((640, 3328), (640, 3584), (896, 2560), (1152, 2048), (4736, 512)):
         assert X.pick_pair_tile(M, N, 4096) == 0 and X.pick_gemm_config(M, N, 4096, X.EPI_STORE) == (128, 1, 1)
+    # a tuned configuration is one of single CTAs and counts for many rows too
+    X.GEMM_TUNING[(2048, 6144, 4096, X.EPI_STORE)] = (256, 1, 1)
+    try:
+        assert X.pick_pair_tile(2048, 6144, 4096) == 0 and X.pick_pair_tile(2048, 6144, 4096, 128, X.EPI_SWIGLU) == 256
+        assert X.pick_gemm_config(2048, 6144, 4096, X.EPI_STORE) == (256, 1, 1)
+    finally:
+        X.GEMM_TUNING.clear()
     # attention: one wave of CTAs; 32 query tiles x heads leave 4 key splits, a shard with one KV head gets 16
     assert X.attn_splits_for(128, 32, 8, 2700) == 4
     assert X.attn_splits_for(128, 4, 1, 2700) == 16
