@@ -59,8 +59,10 @@ constexpr int attn_tc_smem(int mode) { return kSmemQ + attn_stages(mode) * kStag
 // Key splits that merge inside a cluster (portable cluster size); the chunk receive area must fit the dead
 // K/V stages + P buffers, the (max, sum) pairs the dead Q tile.
 constexpr int kMaxClusterSplits = 8;
-static_assert(kMaxClusterSplits * 16384 <= attn_stages(kPlain) * kStageKV + 2 * kSmemP, "chunk receive area");
-static_assert(3 * 2 * 16384 <= attn_stages(kPlain) * kStageKV + 2 * kSmemP, "chunk receive area, 3 splits own 2 chunks each");
+constexpr bool merge_fits(int mode) {        // 3 splits own 2 chunks each
+  return kMaxClusterSplits * 16384 <= attn_stages(mode) * kStageKV + 2 * kSmemP && 3 * 2 * 16384 <= attn_stages(mode) * kStageKV + 2 * kSmemP;
+}
+static_assert(merge_fits(kPlain) && merge_fits(kPooled), "chunk receive area of the forms that merge in a cluster");
 static_assert(kMaxClusterSplits * TROWS * 8 <= kSmemQ, "(max, sum) receive area");
 
 // kPlain, kTwo: tensor maps of the pools.  Head h's slot s is row h * head_rows + s, from column h * head_cols.
@@ -1007,7 +1009,8 @@ extern "C" int js_attn_tc_max_active_clusters(int G, int splits) {
   using namespace js;
   if (splits < 1 || splits > kMaxClusterSplits) return -1;
   const void* kern = nullptr;
-  constexpr int kAttnTcSmem = attn_tc_smem(kPlain);      // what kPooled takes as well
+  constexpr int kAttnTcSmem = attn_tc_smem(kPlain);      // kPooled takes less: as many of its clusters fit, at least
+  static_assert(attn_tc_smem(kPooled) <= attn_tc_smem(kPlain), "the residency asked for is a lower bound");
   switch (G) {
     case 1: kern = reinterpret_cast<const void*>(paged_tree_attn_tc_kernel<1, kPlain>); break;
     case 2: kern = reinterpret_cast<const void*>(paged_tree_attn_tc_kernel<2, kPlain>); break;

@@ -8,6 +8,7 @@
 
 namespace js {
 
+constexpr int kSms = 148;       // of the device this is written for
 constexpr int BM = 128;
 constexpr int BK = 64;          // 64 bf16 = one 128-byte swizzle row
 constexpr int UMMA_K = 16;

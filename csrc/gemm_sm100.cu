@@ -59,7 +59,7 @@ JS_DEVICE unsigned long long gtime() {
 // BUDGET_KB bounds the pipeline's shared memory: ~96 KB lets two CTAs share an SM (more tiles
 // in flight, natural load balance when the tile count is not a multiple of 148), ~192 KB gives
 // one CTA per SM a deeper pipeline.
-// MT = row tiles per CTA (1 or 2): with 2, one CTA computes a 256 x BN tile as two 128-row accumulators that share
+// MT = row tiles per CTA (1 or 2; 2 on request only, CTA pairs are faster): with 2, one CTA computes a 256 x BN tile as two 128-row accumulators that share
 // every weight stage, so a k-block brings 1.5x the FLOPs per byte through the L2-to-SM path (many-row GEMMs).
 // AR = activation rows a stage holds (16, 32 or all 128), for launches of one row tile with at most that many rows: the MMA
 // still reads 128 rows from the start of a stage's activations and meets the stage's weights behind them, which only
@@ -896,7 +896,7 @@ static int launch_few_rows(const ActMaps& ta, const CUtensorMap& tw, const GemmP
 // C = A[M,K] * W[N,K]^T.  epi: 0 store(+residual) 1 swiglu 2 argmax partials 3 top-8 + lse partials 4 fp32 store.
 // bn in {64,128,256} (SwiGLU also 192: 128 tiles of a 24576-wide gate/up fill one wave); split = K-split cluster size (1..4; store/swiglu only); deep selects the pipeline's
 // shared-memory budget: 0 = 96 KB (two CTAs per SM), 2 = 128 KB, 1 = 192 KB (one CTA per SM), 3 = 192 KB with two
-// 128-row tiles per CTA sharing each weight stage (bn 256, no split).
+// 128-row tiles per CTA sharing each weight stage (bn 256, no split; on request only, the measured twin of CTA pairs).
 // Returns 0 or a negative code.
 extern "C" int js_gemm_bf16(const void* A, const void* W, void* C, const void* residual, int M, int N, int K, int lda,
                             int ldw, int ldc, int epi, int bn, int split, int deep, float* part_val, int* part_idx,
@@ -964,7 +964,7 @@ extern "C" int js_gemm_bf16_allreduce(const void* A, const void* W, void* C, con
   const int ctas = ((N + 127) / 128) * ((M + BM - 1) / BM) * split;
   if (push_only < 2) {                                    // the cell modes use neither counters nor waits in the GEMM
     if (ctas > n_flags) return -20;
-    if (push_only == 0 && ctas > (split > 1 ? 148 : 2 * 148)) return -21;   // CTAs that wait for peers must all be resident
+    if (push_only == 0 && ctas > (split > 1 ? kSms : 2 * kSms)) return -21;   // CTAs that wait for peers must all be resident
   }
   if (push_only == 3 && (N % (8 * world)) != 0) return -23;
   CUtensorMap ta, tw;
@@ -1066,7 +1066,7 @@ extern "C" int js_gemm_nvfp4(const void* Aq, const void* sfa, const float* row_s
   // More tiles than SMs: three stages (108 KB, 256 tensor-memory columns), so that two CTAs share an SM and one's
   // epilogue runs under the other's loads.  192 tiles of a 24576 x 4096 gate/up ran as two rounds of one CTA per SM: 30.1 us
   // at 64 rows, 16.4 this way; 325 and 155 at 2048 rows.
-  const bool shared_sm = split == 1 && ((N + 127) / 128) * ((M + BM - 1) / BM) > 148;
+  const bool shared_sm = split == 1 && ((N + 127) / 128) * ((M + BM - 1) / BM) > kSms;
 #define JS_CASE4(EPI_)                                                                                   \
   if (epi == EPI_)                                                                                        \
     return split > 1   ? launch_gemm<128, EPI_, 128, true>(ta, tw, p, split, pdl != 0, stream)            \
@@ -1093,7 +1093,7 @@ extern "C" int js_gemm_nvfp4_allreduce(const void* Aq, const void* sfa, const fl
   const int ctas = ((N + 127) / 128) * ((M + BM - 1) / BM) * split;
   if (push_only < 2) {
     if (ctas > n_flags) return -20;
-    if (push_only == 0 && ctas > 148) return -21;           // CTAs that wait for peers must all be resident
+    if (push_only == 0 && ctas > kSms) return -21;           // CTAs that wait for peers must all be resident
   }
   if (push_only == 3 && (N % (8 * world)) != 0) return -23;
   CUtensorMap ta, tw;
