@@ -46,19 +46,19 @@ def case_gemm(reps: int = 2):
 
 
 def case_gemm_rows2048(reps: int = 2):
-    """The same four shapes at 2048 rows (16 requests x 128 tree nodes, or a prefill chunk), picked configurations:
-    256-column tiles, two row tiles per CTA for o_proj / down_proj, 256-interleaved gate/up."""
+    """The same four shapes at 2048 rows (16 requests x 128 tree nodes, or a prefill chunk) as picked:
+    tiles of 256 rows on CTA pairs."""
     M, H, I = 2048, 4096, 12288
     x, a = bf(M, H), bf(M, I)
     g, u = bf(I, H, scale=0.02), bf(I, H, scale=0.02)
-    w = {"qkv": bf(6144, H, scale=0.02), "o": bf(H, H, scale=0.02), "gu": X.interleave_gate_up(g, u, 256),
+    w = {"qkv": bf(6144, H, scale=0.02), "o": bf(H, H, scale=0.02), "gu": X.interleave_gate_up(g, u),
          "down": bf(H, I, scale=0.02)}
     del g, u
     res = bf(M, H)
     for _ in range(reps):
         X.gemm(x, w["qkv"])
         X.gemm(x, w["o"], out=res, residual=res)
-        X.gemm(x, w["gu"], epi=X.EPI_SWIGLU, bn=256, split=1, deep=0)
+        X.gemm(x, w["gu"], epi=X.EPI_SWIGLU)
         X.gemm(a, w["down"], out=res, residual=res)
     torch.cuda.synchronize()
 
