@@ -413,6 +413,33 @@ def test_paged_attention_of_two_softmax_groups(ext, Hq, Hkv, splits, causal):
     ext.check_status("cuda")
 
 
+@pytest.mark.parametrize("splits", [1, 3])
+@pytest.mark.parametrize("moved", [0, 1, 7])
+def test_attention_over_pages(ext, splits, moved):
+    """Slots as a page table gives them: 16 neighbours a page, which the loaders take as one box, and a few slots of the last pages
+    moved (an accepted path), so that some warps of a tile take a box and others gather; a page at the very end of the pool."""
+    from jetspec_b200.ops import reference as ref
+    pasts, ns, G, H, S = [130, 0, 500, 61], [20, 16, 1, 40], 2, 8, 1024
+    B, T = len(ns), sum(ns)
+    q, kp, vp = rnd(T, H, 128, seed=101), rnd(G, S, 128, seed=102), rnd(G, S, 128, seed=103)
+    pages = torch.randperm(S // 16, generator=torch.Generator().manual_seed(moved)).tolist()
+    pages.remove(S // 16 - 1)
+    smap = torch.zeros(B, 640, dtype=torch.int32)
+    for b in range(B):
+        L = pasts[b] + ns[b]
+        own = [S // 16 - 1] if b == 1 else [pages.pop() for _ in range((L + 15) // 16)]
+        s = torch.tensor([p * 16 + i for p in own for i in range(16)], dtype=torch.int32)[:L]
+        for m in range(min(moved, L // 2)):
+            s[[L - 1 - m, L // 2 - m]] = s[[L // 2 - m, L - 1 - m]]
+        smap[b, :L] = s
+    smap = smap.cuda()
+    cu = torch.tensor([0] + torch.tensor(ns).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+    rows, past = torch.arange(B, dtype=torch.int32, device="cuda"), torch.tensor(pasts, dtype=torch.int32, device="cuda")
+    out = ext.paged_tree_attention(q, kp, vp, smap, rows, cu, past, None, 0.1, True, max(ns), splits=splits, impl="tc")
+    assert rel_err(out, ref.paged_tree_attention(q.float(), kp.float(), vp.float(), smap, rows, cu, past, None, 0.1, True)) < BF16_TOL
+    ext.check_status("cuda")
+
+
 @pytest.mark.parametrize("lens", [[2900] + [30] * 9, [700, 3, 650], [1] * 40, list(range(1, 400, 17))])
 def test_batch_of_unequal_lengths(ext, lens):
     """One new token of each of many sequences, key splits as picked for the batch: splits without a key tile, merged by a launch."""

@@ -137,6 +137,25 @@ def test_gemm_nvfp4_matches_dequantised_product(ext, M, N, K, split):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K", [(100, 19200, 256), (600, 4864, 512), (1100, 4864, 1280), (129, 9600, 768)])
+def test_gemm_nvfp4_with_two_ctas_on_an_sm(ext, M, N, K):
+    """More 128 x 128 tiles than SMs: three stages and 256 tensor-memory columns per CTA, two CTAs side by side and several rounds of
+    them, fewer and more k-blocks than stages, a ragged last row tile; every epilogue."""
+    assert (M + 127) // 128 * (N // 128) > ext.SM_COUNT
+    x, res, qw = _rnd(M, K, seed=10), _rnd(M, N, seed=11), quantize_nvfp4(_rnd(N, K, scale=0.05, seed=12).float())
+    ref = nvfp4_linear_reference(x, qw)
+    err = lambda a, b: float((a.float() - b).abs().max() / b.abs().max())
+    assert err(ext.gemm_nvfp4(x, qw, split=1), ref) < 8e-3
+    assert err(ext.gemm_nvfp4(x, qw, residual=res, split=1), ref + res.float()) < 8e-3
+    assert err(ext.gemm_nvfp4(x, qw, epi=ext.EPI_STORE_F32, split=1), ref) < 1e-3
+    y = ref.view(M, N // 128, 2, 64)
+    want = (torch.nn.functional.silu(y[:, :, 0]) * y[:, :, 1]).reshape(M, N // 2)
+    assert err(ext.gemm_nvfp4(x, qw, epi=ext.EPI_SWIGLU, split=1), want) < 8e-3
+    torch.cuda.synchronize()
+    ext.check_status("cuda")
+
+
+@pytest.mark.gpu
 def test_gemm_nvfp4_epilogues(ext):
     M, H, I = 100, 1024, 1536
     x, res = _rnd(M, H, seed=5), _rnd(M, H, seed=6)
